@@ -1660,25 +1660,49 @@ __global__ void __launch_bounds__(kWide, 1) k_pcg_persist(PcgP P) {
 }
 
 // ---------------------------------------------------------------------------
-// Shared-memory-resident persistent Jacobi-PCG.  CTA b owns the contiguous
-// chunks [c0, c1) (nodes [n0, n1), at most kSmemChunks chunks) and keeps
-// x, r, q, diag, p_new of its nodes and a window [n0-H, n1+H) of w and p
-// (H = nny+1, the reach of a 3x3 stencil) in shared memory for the whole
-// solve.  Per iteration only the H-wide boundary strips of w and p cross
-// L2: published before the second barrier, read after it.  Same chunk
-// partials and canonical sums as the other PCG kernels, so the same bits.
+// On-chip persistent Jacobi-PCG.  CTA b owns the contiguous chunks [c0, c1)
+// (nodes [n0, n1)); a group of 256 threads owns NCH chunks, four nodes of
+// each a thread (the canonical items t, t+256, t+512, t+768), and keeps r, q
+// and w of its nodes in registers for the whole solve, x and diag too (in
+// shared memory for more than two chunks, where the registers run out).  The
+// direction p lives in a shared-memory window [n0-H, n1+H) (H = nny+1, the
+// reach of a 3x3 stencil); the owner forms p = w + beta p for the window's
+// halo itself, from the neighbours' w, so only w crosses CTAs.
+//
+// What bounds it is the latency of the two all-reduces an iteration needs,
+// not bandwidth (the vectors never leave the SM).  They use no grid barrier:
+// every chunk partial, and every w of a boundary strip, is published as a
+// tagged value -- two 64-bit words, each half of the double beside the
+// iteration's 32-bit tag -- and the readers poll the value itself with
+// relaxed loads until both tags match.  One trip through L2 carries arrival
+// and data (a barrier, its error word and the partials behind it were four),
+// and without acquire loads or fences L1 keeps the explicit rows.  A word is
+// not overwritten before its readers have it: iteration i+1 publishes only
+// after the all-reduce that every CTA enters after reading iteration i.
+// Tags go on from solve to solve, so nothing is cleared between them.
+//
+// 12.6 -> 7.0 us an iteration at 513^2 nodes (two chunks a CTA), 9.3 -> 6.0
+// at 65^2 (five CTAs) against the grid-barrier form with the chunk staged in
+// shared memory; same chunk partials and canonical sums, so the same bits.
 // ---------------------------------------------------------------------------
-constexpr int kSmemChunks = 2;
+constexpr int kPcgMaxGroups = 4;   // thread groups (256 threads each) of a CTA
+
+// a partial has a 128-byte line of its own: with eight to a line the pollers
+// of one held up the writers of the others (4,400 against 2,400 cycles an
+// all-reduce of 148 CTAs, 1,750 against 1,850 with 27)
+constexpr int kSlot = 8;
 
 struct PcgS {
   PcgK k;
-  double *w_g, *p_g;      // boundary-strip exchange (full-grid arrays)
-  double *partA, *partB;
-  unsigned int *bar;
+  ulonglong2 *strip;      // [nn] tagged w of the boundary strips
+  ulonglong2 *slotA;      // [nb + 1][kSlot] tagged p.q partials (the last slot is never written)
+  ulonglong2 *slotB;      // [nb + 1][kSlot] tagged r.r and r.w partials
+  unsigned tag;           // tag of the first iteration
   int *bar_err;
   long long spin_limit;
-  unsigned int bar_extra;
+  unsigned int bar_extra; // partials expected beyond the chunks (0; 1 only to test the timeout)
   int H;                  // halo width in nodes
+  int cpc;                // chunks per CTA at most
 };
 
 __host__ __device__ inline void smem_range(int b, int G, int nb, int *c0, int *c1) {
@@ -1686,144 +1710,271 @@ __host__ __device__ inline void smem_range(int b, int G, int nb, int *c0, int *c
   *c1 = (int)((int64_t)(b + 1) * nb / G);
 }
 
-__global__ void __launch_bounds__(kWide, 1) k_pcg_smem(PcgS P) {
+__device__ __forceinline__ void st_tagged(ulonglong2 *p, double v, unsigned tag) {
+  const unsigned long long t = (unsigned long long)tag << 32;
+  const unsigned long long a = t | (unsigned)__double2hiint(v), b = t | (unsigned)__double2loint(v);
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+
+__device__ __forceinline__ bool ld_tagged(const ulonglong2 *p, unsigned tag, double &v) {
+  unsigned long long a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  v = __hiloint2double((int)(unsigned)a, (int)(unsigned)b);
+  return (unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag;
+}
+
+// Polls NV adjacent tagged values per lane that wants some; called by whole
+// warps, which leave together (lanes that left one by one came together
+// again, at the next shuffle, only thousands of cycles later).  Gives up
+// after `limit` polls (recording it in *err) or soon after another warp did.
+template <int NV>
+__device__ __forceinline__ bool poll_tagged(bool want, const ulonglong2 *p, unsigned tag, double *v, int *err,
+                                            long long limit) {
+#pragma unroll
+  for (int q = 0; q < NV; ++q) v[q] = 0.0;
+  for (long long spins = 0;;) {
+    bool got = true;
+    if (want) {
+#pragma unroll
+      for (int q = 0; q < NV; ++q) got &= ld_tagged(p + q, tag, v[q]);
+    }
+    if (__all_sync(0xffffffffu, got)) return true;
+    bool stop = false;
+    if (++spins > limit) {
+      if (!got) atomicExch(err, 1);
+      stop = true;
+    } else if ((spins & 1023) == 0) {
+      stop = *(volatile int *)err != 0;
+    }
+    if (__any_sync(0xffffffffu, stop)) return false;
+  }
+}
+
+// A p at one node of the window; i: the node's slot.  The coefficients and
+// their order are row_apply's.
+__device__ __forceinline__ double row_apply_win(const PcgK &k, int kind, const double *win, int i, int64_t wbase) {
+  if (kind < 0) return 0.0;
+  double acc = 0.0;
+  if (kind < k.n_mat) {
+    const double *w = win + (i - k.nny - 1);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) acc = fma(c_stencil[kind][3 * a + c], w[a * k.nny + c], acc);
+  } else {
+    const int rix = kind - k.n_mat;
+    const int cnt = k.ex_cnt[rix];
+    int32_t col[9];
+    double val[9], xv[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      col[q] = k.ex_col[9 * (size_t)rix + q];
+      val[q] = k.ex_val[9 * (size_t)rix + q];
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) xv[q] = win[(int)(col[q] - wbase)];
+#pragma unroll
+    for (int q = 0; q < 9; ++q)
+      if (q < cnt) acc = fma(val[q], xv[q], acc);
+  }
+  return acc;
+}
+
+// The sum of the chunk partials in the canonical order, in every thread: the
+// first 256 threads poll the slots (b = t, t + 256, ...), then the butterfly
+// and the warp sums in order.  ws: its own shared array per call site.
+// False in every thread when any thread of the CTA gave up.
+template <int NV>
+__device__ __forceinline__ bool sum_slots(const PcgS &P, const ulonglong2 *slots, unsigned tag, int nb, bool ok,
+                                          double (*ws)[PIC_RED_THREADS / 32], double *out) {
+  if (threadIdx.x < PIC_RED_THREADS) {
+    double a[NV], v[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) a[q] = 0.0;
+    for (int b0 = 0; b0 < nb; b0 += PIC_RED_THREADS) {
+      const int b = b0 + threadIdx.x;
+      ok = ok && poll_tagged<NV>(b < nb, slots + (size_t)kSlot * b, tag, v, P.bar_err, P.spin_limit);
+      if (b < nb)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) a[q] = a[q] + v[q];
+    }
+    if (P.bar_extra && threadIdx.x < 32)  // a partial that never comes (failure-path test)
+      ok = ok && poll_tagged<NV>(threadIdx.x == 0, slots + (size_t)kSlot * nb, tag, v, P.bar_err, P.spin_limit);
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      for (int off = 16; off > 0; off >>= 1) a[q] = a[q] + __shfl_xor_sync(0xffffffffu, a[q], off);
+      if ((threadIdx.x & 31) == 0) ws[q][threadIdx.x >> 5] = a[q];
+    }
+  }
+  if (__syncthreads_or(!ok)) return false;
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < PIC_RED_THREADS / 32; ++w) t = t + ws[q][w];
+    out[q] = t;
+  }
+  return true;
+}
+
+template <int NG, int NCH>
+__global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
   extern __shared__ double smem[];
+  constexpr int NI = 4 * NCH;                   // nodes of a thread
+  constexpr bool kSpill = NG * NCH > 2;         // x and diag in shared memory
+  constexpr int NW = PIC_RED_THREADS / 32;
+  __shared__ double wsA[NG * NCH][NW], wsB[NG * NCH][2][NW], wsTA[1][NW], wsTB[2][NW];
   const PcgK &k = P.k;
   PcgState *S = k.st;
   int c0, c1;
   smem_range(blockIdx.x, gridDim.x, k.nb, &c0, &c1);
   const int64_t n0 = (int64_t)c0 * kWide;
   const int64_t n1 = min((int64_t)c1 * kWide, k.nn);
-  const int L = (int)(n1 - n0);
-  const int H = P.H;
+  const int L = (int)(n1 - n0), H = P.H;
   const int64_t wbase = n0 - H;     // node of window slot 0
-  const int W = L + 2 * H;
-  double *win_w = smem, *win_p = win_w + W;
-  double *s_x = win_p + W, *s_r = s_x + kSmemChunks * kWide, *s_q = s_r + kSmemChunks * kWide;
-  double *s_d = s_q + kSmemChunks * kWide, *s_pn = s_d + kSmemChunks * kWide;
-  // load own x, r, diag and the window of w (p is not read before iteration 1)
-  for (int i = threadIdx.x; i < L; i += kWide) {
-    s_x[i] = __ldcg(k.x + n0 + i);
-    s_r[i] = __ldcg(k.r + n0 + i);
-    s_d[i] = k.diag[n0 + i];
+  double *win = smem;               // [cpc*kWide + 2H] p
+  double *halo = win + P.cpc * kWide + 2 * H;  // [2H] w of the halo
+  double *s_x = halo + 2 * H, *s_d = s_x + P.cpc * kWide;  // kSpill only
+  const int grp = threadIdx.x / PIC_RED_THREADS, t = threadIdx.x % PIC_RED_THREADS;
+  const int lane = threadIdx.x & 31, gw = t >> 5;
+  // own nodes: item it of chunk h at offset off(h, it) from n0
+  auto off = [&](int u) { return ((u >> 2) * NG + grp) * kWide + (u & 3) * PIC_RED_THREADS + t; };
+  double x[kSpill ? 1 : NI], d[kSpill ? 1 : NI], r[NI], w[NI], q[NI];
+  int kind[NI];
+#pragma unroll
+  for (int u = 0; u < NI; ++u) {
+    const int o = off(u);
+    const bool in = o < L;
+    const int64_t n = n0 + o;
+    const double xv = in ? __ldcg(k.x + n) : 0.0, dv = in ? k.diag[n] : 1.0;
+    if constexpr (kSpill) {
+      if (in) {
+        s_x[o] = xv;
+        s_d[o] = dv;
+      }
+    } else {
+      x[u] = xv;
+      d[u] = dv;
+    }
+    r[u] = in ? __ldcg(k.r + n) : 0.0;
+    w[u] = in ? __ldcg(k.w + n) : 0.0;
+    q[u] = 0.0;
+    kind[u] = in ? k.row_kind[n] : -1;
   }
-  for (int i = threadIdx.x; i < W; i += kWide) {
-    int64_t m = wbase + i;
-    win_w[i] = (m >= 0 && m < k.nn) ? __ldcg(k.w + m) : 0.0;
-    win_p[i] = 0.0;
+  for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) {
+    const int64_t m = wbase + (i < H ? i : L + i);
+    halo[i] = (m >= 0 && m < k.nn) ? __ldcg(k.w + m) : 0.0;
   }
+  for (int i = threadIdx.x; i < L + 2 * H; i += blockDim.x) win[i] = 0.0;
   __syncthreads();
-  double rho = __ldcg(&S->rho), normRHS = __ldcg(&S->normRHS);
-  const double tol2 = S->tol2;
+  double rho = __ldcg(&S->rho);
+  const double normRHS = __ldcg(&S->normRHS), tol2 = S->tol2;
   const int maxit = S->maxit;
   int done = __ldcg(&S->done), iter = 0, ierr = 0;
   double beta = 0.0, normR = 0.0, rho0 = 0.0;
   bool ok = true;
   while (!done) {
     const bool first = iter == 0;
-    auto pn = [&](int64_t m) {
-      const int64_t i = m - wbase;
-      return first ? win_w[i] : fma(beta, win_p[i], win_w[i]);
-    };
-    // (A) p = w + beta p, q = A p, chunk partials of p.q
-    for (int c = c0; c < c1; ++c) {
-      const int off = (c - c0) * kWide;
-      const int nvalid = (int)min((int64_t)kWide, n1 - (int64_t)c * kWide);
-      const int64_t n = (int64_t)c * kWide + threadIdx.x;
-      double pv = 0.0, qv = 0.0;
-      if (threadIdx.x < nvalid) {
-        pv = pn(n);
-        qv = row_apply(k, n, pn);
-      }
-      s_pn[off + threadIdx.x] = pv;
-      s_q[off + threadIdx.x] = qv;
-      __syncthreads();
-      double part[1];
-      const double(*a)[kWide] = reinterpret_cast<const double(*)[kWide]>(s_pn + off);
-      const double(*b)[kWide] = reinterpret_cast<const double(*)[kWide]>(s_q + off);
-      chunk_dots<1>(a, b, nvalid, part);
-      if (threadIdx.x == 0) P.partA[c] = part[0];
+    const unsigned tag = P.tag + (unsigned)iter;
+    // (A) p = w + beta p on the window, q = A p, chunk partials of p.q
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {
+      const int o = off(u);
+      if (o < L) win[H + o] = first ? w[u] : fma(beta, win[H + o], w[u]);
     }
-    if (!(ok = grid_barrier(P.bar, P.bar_err, P.spin_limit, P.bar_extra))) break;
+    for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) {
+      const int slot = i < H ? i : L + i;
+      win[slot] = first ? halo[i] : fma(beta, win[slot], halo[i]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < NCH; ++h) {
+      double acc = 0.0;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int u = 4 * h + it, o = off(u);
+        if (o < L) {
+          q[u] = row_apply_win(k, kind[u], win, H + o, wbase);
+          acc = fma(win[H + o], q[u], acc);
+        }
+      }
+      for (int s = 16; s > 0; s >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, s);
+      if (lane == 0) wsA[h * NG + grp][gw] = acc;
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(PIC_RED_THREADS) : "memory");
+    if (t < NCH) {
+      const int c = c0 + t * NG + grp;
+      if (c < c1) {
+        double s = 0.0;
+#pragma unroll
+        for (int v = 0; v < NW; ++v) s = s + wsA[t * NG + grp][v];
+        st_tagged(P.slotA + (size_t)kSlot * c, s, tag);
+      }
+    }
+    __syncwarp();
     double pq;
-    final_sum_wide<1>(P.partA, k.nb, &pq);
+    if (!(ok = sum_slots<1>(P, P.slotA, tag, k.nb, true, wsTA, &pq))) break;
     if (pq == 0.0) {
       ierr = 3;
       break;
     }
     const double alpha = rho / pq;
-    // (B) x += alpha p, r -= alpha q, w = r/diag; window gets w and p for the
-    // next iteration; boundary strips are published to L2
-    for (int c = c0; c < c1; ++c) {
-      const int off = (c - c0) * kWide;
-      const int nvalid = (int)min((int64_t)kWide, n1 - (int64_t)c * kWide);
-      const int i = off + threadIdx.x;
-      if (threadIdx.x < nvalid) {
-        const double pv = s_pn[i];
-        s_x[i] = fma(alpha, pv, s_x[i]);
-        const double rv = fma(-alpha, s_q[i], s_r[i]);
-        const double wv = rv / s_d[i];
-        s_r[i] = rv;
-        s_q[i] = wv;  // q is dead after the update: reuse its slot for w
-        win_w[H + i] = wv;
-        win_p[H + i] = pv;
-        if (i < H || i >= L - H) {
-          P.w_g[n0 + i] = wv;
-          P.p_g[n0 + i] = pv;
+    // (B) x += alpha p, r -= alpha q, w = r/diag; the strips the neighbours
+    // need; chunk partials of r.r and r.w
+#pragma unroll
+    for (int h = 0; h < NCH; ++h) {
+      double arr = 0.0, arw = 0.0;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int u = 4 * h + it, o = off(u);
+        if (o < L) {
+          r[u] = fma(-alpha, q[u], r[u]);
+          if constexpr (kSpill) w[u] = r[u] / s_d[o];
+          else w[u] = r[u] / d[u];
+          if (o < H || o >= L - H) st_tagged(P.strip + n0 + o, w[u], tag);
+          arr = fma(r[u], r[u], arr);
+          arw = fma(r[u], w[u], arw);
         }
       }
-      __syncthreads();
-      double part[2];
-      const double *ra = s_r + off;
-      const double *wa = s_q + off;
-      // r.r and r.w in one canonical pass
-      {
-        __shared__ double ws2[2][PIC_RED_THREADS / 32];
-        if (threadIdx.x < PIC_RED_THREADS) {
-          double arr = 0.0, arw = 0.0;
-          for (int it = 0; it < PIC_RED_ITEMS; ++it) {
-            int j = it * PIC_RED_THREADS + threadIdx.x;
-            if (j < nvalid) {
-              arr = fma(ra[j], ra[j], arr);
-              arw = fma(ra[j], wa[j], arw);
-            }
-          }
-          for (int o2 = 16; o2 > 0; o2 >>= 1) {
-            arr = arr + __shfl_xor_sync(0xffffffffu, arr, o2);
-            arw = arw + __shfl_xor_sync(0xffffffffu, arw, o2);
-          }
-          if ((threadIdx.x & 31) == 0) {
-            ws2[0][threadIdx.x >> 5] = arr;
-            ws2[1][threadIdx.x >> 5] = arw;
-          }
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          double t0 = 0.0, t1 = 0.0;
-          for (int q = 0; q < PIC_RED_THREADS / 32; ++q) {
-            t0 = t0 + ws2[0][q];
-            t1 = t1 + ws2[1][q];
-          }
-          part[0] = t0;
-          part[1] = t1;
-          P.partB[c] = part[0];
-          P.partB[k.nb + c] = part[1];
-        }
-        __syncthreads();
+      for (int s = 16; s > 0; s >>= 1) {
+        arr = arr + __shfl_xor_sync(0xffffffffu, arr, s);
+        arw = arw + __shfl_xor_sync(0xffffffffu, arw, s);
+      }
+      if (lane == 0) {
+        wsB[h * NG + grp][0][gw] = arr;
+        wsB[h * NG + grp][1][gw] = arw;
       }
     }
-    if (!(ok = grid_barrier(P.bar, P.bar_err, P.spin_limit, P.bar_extra))) break;
-    // halo of the window from the neighbours' published strips
-    for (int i = threadIdx.x; i < 2 * H; i += kWide) {
-      const int slot = (i < H) ? i : (L + i);
-      const int64_t m = wbase + slot;
-      if (m >= 0 && m < k.nn) {
-        win_w[slot] = __ldcg(P.w_g + m);
-        win_p[slot] = __ldcg(P.p_g + m);
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(PIC_RED_THREADS) : "memory");
+    if (t < 2 * NCH) {
+      const int h = t >> 1, c = c0 + h * NG + grp;
+      if (c < c1) {
+        double s = 0.0;
+#pragma unroll
+        for (int v = 0; v < NW; ++v) s = s + wsB[h * NG + grp][t & 1][v];
+        st_tagged(P.slotB + (size_t)kSlot * c + (t & 1), s, tag);
       }
+    }
+    __syncwarp();
+    // off the path of the reductions: x, and the halo of w
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {
+      const int o = off(u);
+      if (o < L) {
+        if constexpr (kSpill) s_x[o] = fma(alpha, win[H + o], s_x[o]);
+        else x[u] = fma(alpha, win[H + o], x[u]);
+      }
+    }
+    for (int i0 = 0; i0 < 2 * H; i0 += blockDim.x) {
+      const int i = i0 + threadIdx.x;
+      const int64_t m = wbase + (i < H ? i : L + i);
+      const bool want = i < 2 * H && m >= 0 && m < k.nn;
+      double v;
+      ok = ok && poll_tagged<1>(want, P.strip + m, tag, &v, P.bar_err, P.spin_limit);
+      if (want) halo[i] = v;
     }
     double tot[2];
-    final_sum_wide<2>(P.partB, k.nb, tot);
+    if (!(ok = sum_slots<2>(P, P.slotB, tag, k.nb, ok, wsTB, tot))) break;
     normR = tot[0];
     rho0 = rho;
     rho = tot[1];
@@ -1833,7 +1984,14 @@ __global__ void __launch_bounds__(kWide, 1) k_pcg_smem(PcgS P) {
     else if (rho0 == 0.0) { ierr = 2; done = 1; }
     else beta = rho / rho0;
   }
-  for (int i = threadIdx.x; i < L; i += kWide) k.x[n0 + i] = s_x[i];
+#pragma unroll
+  for (int u = 0; u < NI; ++u) {
+    const int o = off(u);
+    if (o < L) {
+      if constexpr (kSpill) k.x[n0 + o] = s_x[o];
+      else k.x[n0 + o] = x[u];
+    }
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     S->iter = iter;
     S->ierr = ok ? ierr : 4;
@@ -2806,6 +2964,7 @@ static void free_all() {
   F(g.d_ex_val); F(g.d_ex_val32); F(g.d_fcg32); F(g.d_diag); F(g.d_ppr_kind); F(g.d_ppr_ptr); F(g.d_ppr_nodes); F(g.d_ppr_rows);
   F(g.d_ppr_h); F(g.d_phi); F(g.d_rho); F(g.d_efx); F(g.d_efy); F(g.d_efxy); F(g.d_coef); F(g.d_coef32); F(g.d_b); F(g.d_x);
   F(g.d_r); F(g.d_w); F(g.d_p[0]); F(g.d_p[1]); F(g.d_q); F(g.d_part); F(g.d_pcg); F(g.d_bar);
+  F(g.d_pcg_slot); F(g.d_pcg_strip);
   F(g.d_z); F(g.d_dot); F(g.d_dot_ticket); F(g.d_fcg); F(g.d_fcg_P); F(g.d_fcg_Q); F(g.d_fcg_part);
   precond_free();
   diag_free();
@@ -3127,6 +3286,37 @@ static int run_rhs() {
   return PIC_OK;
 }
 
+// The on-chip PCG built for the chunks a CTA owns at most: a group of 256
+// threads a chunk while four groups do, then two chunks a group.
+struct SmemPcg {
+  const void *fn;
+  int threads;
+  size_t bytes;  // dynamic shared memory
+};
+
+static SmemPcg smem_pcg(int cpc) {
+  SmemPcg v;
+  const int ng = cpc <= 1 ? 1 : cpc <= 2 ? 2 : kPcgMaxGroups;
+  v.fn = cpc <= 1 ? (const void *)k_pcg_smem<1, 1>
+         : cpc <= 2 ? (const void *)k_pcg_smem<2, 1>
+         : cpc <= 4 ? (const void *)k_pcg_smem<4, 1>
+                    : (const void *)k_pcg_smem<4, 2>;
+  v.threads = 256 * ng;
+  const size_t own = (size_t)cpc * kWide, H = (size_t)g.m.nny + 1;
+  v.bytes = (own + 4 * H + (cpc > 2 ? 2 * own : 0)) * sizeof(double);
+  return v;
+}
+
+// Tags and slots of the on-chip PCG as if no solve had run.
+static int pcg_slots_clear() {
+  if (!g.d_pcg_slot) return PIC_OK;
+  int rc;
+  if ((rc = zero_async(g.d_pcg_slot, 2 * kSlot * (size_t)(g.red_blocks + 1) * sizeof(ulonglong2), g.st))) return rc;
+  if ((rc = zero_async(g.d_pcg_strip, (size_t)g.nn * sizeof(ulonglong2), g.st))) return rc;
+  g.pcg_tag = 1;
+  return PIC_OK;
+}
+
 static int run_pcg(pic_solve_stats *stats) {
   PcgState h;
   std::memset(&h, 0, sizeof h);
@@ -3156,18 +3346,18 @@ static int run_pcg(pic_solve_stats *stats) {
     if (g.smem_grid > 0) {
       PcgS Q;
       Q.k = pcg_k(0);
-      Q.w_g = g.d_p[1];  // strip exchange buffers: free while the smem solver runs
-      Q.p_g = g.d_p[0];
-      Q.partA = P.partA;
-      Q.partB = P.partB;
-      Q.bar = P.bar;
+      Q.strip = g.d_pcg_strip;
+      Q.slotA = g.d_pcg_slot;
+      Q.slotB = g.d_pcg_slot + (size_t)kSlot * (g.red_blocks + 1);
+      Q.tag = g.pcg_tag;
       Q.bar_err = P.bar_err;
       Q.spin_limit = P.spin_limit;
       Q.bar_extra = P.bar_extra;
       Q.H = g.m.nny + 1;
+      Q.cpc = g.smem_cpc;
       void *args[] = {&Q};
-      PIC_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_smem, dim3(g.smem_grid), dim3(kWide), args,
-                                           g.smem_bytes, g.st));
+      const SmemPcg v = smem_pcg(g.smem_cpc);
+      PIC_CUDA(cudaLaunchCooperativeKernel(v.fn, dim3(g.smem_grid), dim3(v.threads), args, g.smem_bytes, g.st));
     } else {
       void *args[] = {&P};
       PIC_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_persist, dim3(g.coop_grid), dim3(kWide),
@@ -3176,7 +3366,9 @@ static int run_pcg(pic_solve_stats *stats) {
     PIC_LAUNCHED();
     PIC_CUDA(cudaMemcpyAsync(&hs, g.d_pcg, sizeof hs, cudaMemcpyDeviceToHost, g.st));
     PIC_CUDA(cudaStreamSynchronize(g.st));
+    if (g.smem_grid > 0) g.pcg_tag += (unsigned)hs.iter + 2;  // every tag this solve can have published
     if (hs.ierr == 4) {
+      if (int rc_ = pcg_slots_clear()) return rc_;
       set_error("pic_ife_solve: PCG grid barrier timed out");
       return PIC_ERR_CUDA;
     }
@@ -4415,23 +4607,26 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     const char *envf = getenv("PIC_FCG_PERSISTENT");
     const bool want_f = !(envf && envf[0] == '0');
     g.fcg_coop_grid = (want_f && coop && per_sm_f > 0) ? std::min(g.red_blocks, per_sm_f * nsm) : 0;
-    // shared-memory-resident variant: every CTA owns at most kSmemChunks
-    // chunks and its window of w and p fits next to them
+    // on-chip variant: at most eight chunks a CTA, whose window of p fits in
+    // shared memory (and x and diag beside it from three chunks on)
     g.smem_grid = 0;
     const char *env2 = getenv("PIC_PCG_SMEM");
     bool want_smem = want && !(env2 && env2[0] == '0');
-    const int H = m.nny + 1;
-    const size_t bytes = (size_t)(2 * (kSmemChunks * kWide + 2 * H) + 5 * kSmemChunks * kWide) * sizeof(double);
     int max_smem = 0;
     PIC_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    if (want_smem && coop && g.ex_local && bytes + 2048 <= (size_t)max_smem) {
-      PIC_CUDA(cudaFuncSetAttribute(k_pcg_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    const int cpc = (g.red_blocks + nsm - 1) / nsm;
+    const SmemPcg v = smem_pcg(cpc);
+    if (want_smem && coop && g.ex_local && cpc <= 2 * kPcgMaxGroups && v.bytes + 4096 <= (size_t)max_smem) {
+      PIC_CUDA(cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.bytes));
       int per_sm2 = 0;
-      PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, k_pcg_smem, kWide, bytes));
-      int G = std::min(g.red_blocks, per_sm2 * nsm);
-      if (per_sm2 > 0 && (int64_t)G * kSmemChunks >= g.red_blocks) {
-        g.smem_grid = G;
-        g.smem_bytes = bytes;
+      PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, v.fn, v.threads, v.bytes));
+      if (per_sm2 > 0) {
+        g.smem_grid = (g.red_blocks + cpc - 1) / cpc;
+        g.smem_cpc = cpc;
+        g.smem_bytes = v.bytes;
+        if ((rc = dalloc(&g.d_pcg_slot, 2 * kSlot * (size_t)(g.red_blocks + 1)))) return rc;
+        if ((rc = dalloc(&g.d_pcg_strip, (size_t)nn))) return rc;
+        if ((rc = pcg_slots_clear())) return rc;
       }
     }
     // failure-path test hooks: a short wait limit and an arrival that never comes
