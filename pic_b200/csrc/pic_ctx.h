@@ -129,6 +129,10 @@ struct Ctx {
   int32_t *d_ex_cnt = nullptr, *d_ex_col = nullptr;  // explicit rows: count + 9 padded slots
   double *d_ex_val = nullptr;
   float *d_ex_val32 = nullptr;     // FP32 copy (inner iterations of the mixed-precision FCG)
+  double *d_st_tab = nullptr;      // or the stencil of every row kind, and its strides
+  float *d_st_tab32 = nullptr;
+  int st_cs = 0, st_rs = 0;
+  bool ex_stencil = true;
   float *d_fcg32 = nullptr;        // mixed-precision FCG: 11 FP32 vectors, allocated on first use
   int fcg_inner32 = 0;             // mixed precision: FP32 inner FCG in FP64 refinement (pic_set_fcg_inner)
   int n_mat = 0;

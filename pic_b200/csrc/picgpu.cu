@@ -20,11 +20,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <map>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "pic_ctx.h"
@@ -1259,6 +1261,11 @@ struct PcgK {
   const int32_t *row_kind, *ex_cnt, *ex_col;
   const double *ex_val, *diag;
   const float *ex_val32;  // FP32 copy of ex_val
+  // stencil of every row kind, coefficient q of kind r at q st_cs + r st_rs
+  // (null: explicit rows are ex_cnt, ex_col, ex_val)
+  const double *st_tab;
+  const float *st_tab32;
+  int st_cs, st_rs;
   double *x, *r, *w, *q, *b;
   const double *p_old;
   double *p_new;
@@ -1271,8 +1278,17 @@ struct PcgK {
   int nb;
 };
 
+// Node of stencil position q of node n, kept inside the vectors: the
+// positions outside the grid carry the coefficient 0.
+__device__ __forceinline__ int64_t stencil_node(const PcgK &k, int64_t n, bool edge, int q) {
+  const int64_t m = n + (int64_t)(q / 3 - 1) * k.nny + (q % 3 - 1);
+  return edge ? (m < 0 ? 0 : m >= k.nn ? k.nn - 1 : m) : m;
+}
+
 // y = A*v on the full grid for a node given a functor that returns v at a node.
-template <class F>
+// EX: explicit rows are column lists (0), stencils (1), or either (2: found at
+// run time; the persistent FCG, at its register limit, is built for each).
+template <int EX = 2, class F>
 __device__ __forceinline__ double row_apply(const PcgK &k, int64_t n, F v) {
   int kind = k.row_kind[n];
   if (kind < 0) return 0.0;
@@ -1283,6 +1299,15 @@ __device__ __forceinline__ double row_apply(const PcgK &k, int64_t n, F v) {
     for (int a = 0; a < 3; ++a)
 #pragma unroll
       for (int c = 0; c < 3; ++c) acc = fma(c_stencil[kind][3 * a + c], v(base + (int64_t)a * k.nny + c), acc);
+  } else if (EX == 1 || (EX == 2 && k.st_tab)) {
+    const bool edge = n < k.nny + 1 || n >= k.nn - k.nny - 1;
+    double val[9], xv[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) val[q] = k.st_tab[q * k.st_cs + kind * k.st_rs];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) xv[q] = v(stencil_node(k, n, edge, q));
+#pragma unroll
+    for (int q = 0; q < 9; ++q) acc = fma(val[q], xv[q], acc);
   } else {
     // explicit row, padded to 9 slots so all loads are in flight together;
     // only the first cnt slots enter the sum, in CSR order
@@ -1681,9 +1706,11 @@ __global__ void __launch_bounds__(kWide, 1) k_pcg_persist(PcgP P) {
 // after the all-reduce that every CTA enters after reading iteration i.
 // Tags go on from solve to solve, so nothing is cleared between them.
 //
-// 12.6 -> 7.0 us an iteration at 513^2 nodes (two chunks a CTA), 9.3 -> 6.0
-// at 65^2 (five CTAs) against the grid-barrier form with the chunk staged in
-// shared memory; same chunk partials and canonical sums, so the same bits.
+// 12.6 -> 6.1 us an iteration at 513^2 nodes (two chunks a CTA), 9.3 -> 3.5
+// at 65^2 (five CTAs), 12.2 -> 3.1 on a 76x51 r-z mesh (explicit rows) against
+// the grid-barrier form with the chunk staged in shared memory; same chunk
+// partials and canonical sums, so the same bits.  Of 6,600 cycles at 65^2 the
+// two exchanges take 4,000, A p 700, the two chunk sums 1,000.
 // ---------------------------------------------------------------------------
 constexpr int kPcgMaxGroups = 4;   // thread groups (256 threads each) of a CTA
 
@@ -1716,27 +1743,31 @@ __device__ __forceinline__ void st_tagged(ulonglong2 *p, double v, unsigned tag)
   asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
 }
 
-__device__ __forceinline__ bool ld_tagged(const ulonglong2 *p, unsigned tag, double &v) {
-  unsigned long long a, b;
-  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-  v = __hiloint2double((int)(unsigned)a, (int)(unsigned)b);
-  return (unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag;
-}
-
-// Polls NV adjacent tagged values per lane that wants some; called by whole
-// warps, which leave together (lanes that left one by one came together
+// Polls N tagged values per lane, those it wants, until every lane of the
+// warp has its own; all loads of a round are in flight together.  Called by
+// whole warps, which leave together (lanes that left one by one came together
 // again, at the next shuffle, only thousands of cycles later).  Gives up
-// after `limit` polls (recording it in *err) or soon after another warp did.
-template <int NV>
-__device__ __forceinline__ bool poll_tagged(bool want, const ulonglong2 *p, unsigned tag, double *v, int *err,
-                                            long long limit) {
-#pragma unroll
-  for (int q = 0; q < NV; ++q) v[q] = 0.0;
+// after `limit` rounds (recording it in *err) or soon after another warp did.
+template <int N>
+__device__ __forceinline__ bool poll_tagged(const bool (&want)[N], const ulonglong2 *const (&p)[N], unsigned tag,
+                                            double (&v)[N], int *err, long long limit) {
   for (long long spins = 0;;) {
-    bool got = true;
-    if (want) {
+    unsigned long long a[N], b[N];
 #pragma unroll
-      for (int q = 0; q < NV; ++q) got &= ld_tagged(p + q, tag, v[q]);
+    for (int q = 0; q < N; ++q) {
+      a[q] = b[q] = (unsigned long long)tag << 32;
+      asm volatile(
+          "{.reg .pred w; setp.ne.u32 w, %3, 0;\n"
+          "@w ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];}"
+          : "+l"(a[q]), "+l"(b[q])
+          : "l"(p[q]), "r"((unsigned)want[q])
+          : "memory");
+    }
+    bool got = true;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      got &= (unsigned)(a[q] >> 32) == tag && (unsigned)(b[q] >> 32) == tag;
+      v[q] = __hiloint2double((int)(unsigned)a[q], (int)(unsigned)b[q]);
     }
     if (__all_sync(0xffffffffu, got)) return true;
     bool stop = false;
@@ -1750,6 +1781,28 @@ __device__ __forceinline__ bool poll_tagged(bool want, const ulonglong2 *p, unsi
   }
 }
 
+// a / d with y = 1/d rounded to nearest (NaN where d is out of the range in
+// which this holds), the same bits as the division: a correction of a y makes
+// it the quotient to within its last place, and by Markstein's theorem (IBM
+// J. Res. Dev. 34, 1990) one more with the exact remainder rounds correctly.
+// Five dependent operations and no branch for the Jacobi preconditioner's
+// divisions by constants; zeros (every Dirichlet node) keep their sign.
+// exact is cleared where the caller has to divide.
+__device__ __forceinline__ double div_const(double a, double d, double y, bool &exact) {
+  double q = a * y;
+  const double zero = q;
+  q = fma(fma(-q, d, a), y, q);
+  q = fma(fma(-q, d, a), y, q);
+  const double m = fabs(a);
+  exact = exact && ((m > 1e-250 && m < 1e250 && y == y) || m == 0.0);
+  return m == 0.0 ? zero : q;
+}
+
+__device__ __forceinline__ double recip_const(double d) {
+  const double m = fabs(d);
+  return m > 1e-40 && m < 1e40 ? 1.0 / d : __longlong_as_double(0x7ff8000000000000ll);
+}
+
 // A p at one node of the window; i: the node's slot.  The coefficients and
 // their order are row_apply's.
 __device__ __forceinline__ double row_apply_win(const PcgK &k, int kind, const double *win, int i, int64_t wbase) {
@@ -1761,6 +1814,13 @@ __device__ __forceinline__ double row_apply_win(const PcgK &k, int kind, const d
     for (int a = 0; a < 3; ++a)
 #pragma unroll
       for (int c = 0; c < 3; ++c) acc = fma(c_stencil[kind][3 * a + c], w[a * k.nny + c], acc);
+  } else if (k.st_tab) {  // the window holds 0 outside the grid
+    const double *w = win + (i - k.nny - 1);
+    double val[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) val[q] = k.st_tab[q * k.st_cs + kind * k.st_rs];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) acc = fma(val[q], w[(q / 3) * k.nny + q % 3], acc);
   } else {
     const int rix = kind - k.n_mat;
     const int cnt = k.ex_cnt[rix];
@@ -1782,24 +1842,59 @@ __device__ __forceinline__ double row_apply_win(const PcgK &k, int kind, const d
 
 // The sum of the chunk partials in the canonical order, in every thread: the
 // first 256 threads poll the slots (b = t, t + 256, ...), then the butterfly
-// and the warp sums in order.  ws: its own shared array per call site.
-// False in every thread when any thread of the CTA gave up.
-template <int NV>
-__device__ __forceinline__ bool sum_slots(const PcgS &P, const ulonglong2 *slots, unsigned tag, int nb, bool ok,
-                                          double (*ws)[PIC_RED_THREADS / 32], double *out) {
-  if (threadIdx.x < PIC_RED_THREADS) {
-    double a[NV], v[NV];
+// and the warp sums in order.  With NH > 0 every thread polls the w of NH nodes
+// of the window's halo in the same round.  ws: its own shared array per call
+// site.  False in every thread when any thread of the CTA gave up.
+template <int NV, int NH>
+__device__ __forceinline__ bool exchange(const PcgS &P, const ulonglong2 *slots, unsigned tag, int nb, int L,
+                                         int64_t wbase, double *halo, double (*ws)[PIC_RED_THREADS / 32],
+                                         double *out) {
+  constexpr int N = NH + 2 * NV;
+  bool ok = true;
+  const int bd = blockDim.x, nh = NH ? 2 * P.H : 0;
+  double a[NV];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) a[q] = 0.0;
-    for (int b0 = 0; b0 < nb; b0 += PIC_RED_THREADS) {
-      const int b = b0 + threadIdx.x;
-      ok = ok && poll_tagged<NV>(b < nb, slots + (size_t)kSlot * b, tag, v, P.bar_err, P.spin_limit);
-      if (b < nb)
+  for (int q = 0; q < NV; ++q) a[q] = 0.0;
+  int i0 = 0, b0 = 0;
+  do {  // one round unless the strips or the slots are very many
+    bool want[N];
+    const ulonglong2 *p[N];
+    double v[N];
 #pragma unroll
-        for (int q = 0; q < NV; ++q) a[q] = a[q] + v[q];
+    for (int q = 0; q < NH; ++q) {
+      const int i = i0 + q * bd + threadIdx.x;
+      const int64_t m = wbase + (i < P.H ? i : L + i);
+      want[q] = i < nh && m >= 0 && m < P.k.nn;
+      p[q] = P.strip + m;
     }
-    if (P.bar_extra && threadIdx.x < 32)  // a partial that never comes (failure-path test)
-      ok = ok && poll_tagged<NV>(threadIdx.x == 0, slots + (size_t)kSlot * nb, tag, v, P.bar_err, P.spin_limit);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int b = b0 + q * PIC_RED_THREADS + threadIdx.x;
+#pragma unroll
+      for (int c = 0; c < NV; ++c) {
+        want[NH + q * NV + c] = threadIdx.x < PIC_RED_THREADS && b < nb;
+        p[NH + q * NV + c] = slots + (size_t)kSlot * b + c;
+      }
+    }
+    ok = ok && poll_tagged<N>(want, p, tag, v, P.bar_err, P.spin_limit);
+#pragma unroll
+    for (int q = 0; q < NH; ++q)
+      if (want[q]) halo[i0 + q * bd + threadIdx.x] = v[q];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+      for (int c = 0; c < NV; ++c)
+        if (want[NH + q * NV + c]) a[c] = a[c] + v[NH + q * NV + c];
+    i0 += NH * bd;
+    b0 += 2 * PIC_RED_THREADS;
+  } while (i0 < nh || b0 < nb);
+  if (P.bar_extra && threadIdx.x < 32) {  // a partial that never comes (failure-path test)
+    const bool want[1] = {threadIdx.x == 0};
+    const ulonglong2 *const p[1] = {slots + (size_t)kSlot * nb};
+    double v[1];
+    ok = ok && poll_tagged<1>(want, p, tag, v, P.bar_err, P.spin_limit);
+  }
+  if (threadIdx.x < PIC_RED_THREADS) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
       for (int off = 16; off > 0; off >>= 1) a[q] = a[q] + __shfl_xor_sync(0xffffffffu, a[q], off);
@@ -1823,6 +1918,10 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
   constexpr int NI = 4 * NCH;                   // nodes of a thread
   constexpr bool kSpill = NG * NCH > 2;         // x and diag in shared memory
   constexpr int NW = PIC_RED_THREADS / 32;
+  // stencil coefficients in registers: every node's (one group), or those of
+  // the thread's first unknown, which most of its nodes share (two groups)
+  constexpr int NC = NG == 1 ? NI : NG == 2 ? 1 : 0;
+  constexpr int NH = NG == 1 ? 2 : NG == 2 ? 3 : 1;  // halo nodes a round: the strips of square grids of their size
   __shared__ double wsA[NG * NCH][NW], wsB[NG * NCH][2][NW], wsTA[1][NW], wsTB[2][NW];
   const PcgK &k = P.k;
   PcgState *S = k.st;
@@ -1839,8 +1938,10 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
   const int lane = threadIdx.x & 31, gw = t >> 5;
   // own nodes: item it of chunk h at offset off(h, it) from n0
   auto off = [&](int u) { return ((u >> 2) * NG + grp) * kWide + (u & 3) * PIC_RED_THREADS + t; };
-  double x[kSpill ? 1 : NI], d[kSpill ? 1 : NI], r[NI], w[NI], q[NI];
-  int kind[NI];
+  constexpr int NR = kSpill ? 1 : NI;
+  double x[NR], d[NR], y[NR], p[NR], r[NI], w[NI], q[NI];
+  double cf[NC ? NC : 1][9];
+  int kind[NI], home = -1;
 #pragma unroll
   for (int u = 0; u < NI; ++u) {
     const int o = off(u);
@@ -1855,12 +1956,28 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
     } else {
       x[u] = xv;
       d[u] = dv;
+      y[u] = recip_const(dv);
+      p[u] = 0.0;
     }
     r[u] = in ? __ldcg(k.r + n) : 0.0;
     w[u] = in ? __ldcg(k.w + n) : 0.0;
     q[u] = 0.0;
     kind[u] = in ? k.row_kind[n] : -1;
+    if (home < 0) home = kind[u];
   }
+  // warps whose rows are all in registers form A p without a load or branch
+  bool fast = NC > 0 && k.st_tab != nullptr;
+  if constexpr (NC > 0) {
+#pragma unroll
+    for (int u = 0; u < NI; ++u) {
+      if (NC == 1) fast = fast && (kind[u] < 0 || kind[u] == home);
+      if (NC == 1 && u > 0) continue;
+      const int kd = NC == 1 ? home : kind[u];
+#pragma unroll
+      for (int c = 0; c < 9; ++c) cf[NC == 1 ? 0 : u][c] = kd >= 0 && k.st_tab ? k.st_tab[c * k.st_cs + kd * k.st_rs] : 0.0;
+    }
+  }
+  fast = __all_sync(0xffffffffu, fast);
   for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) {
     const int64_t m = wbase + (i < H ? i : L + i);
     halo[i] = (m >= 0 && m < k.nn) ? __ldcg(k.w + m) : 0.0;
@@ -1876,29 +1993,70 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
   while (!done) {
     const bool first = iter == 0;
     const unsigned tag = P.tag + (unsigned)iter;
-    // (A) p = w + beta p on the window, q = A p, chunk partials of p.q
+    // (A) p = w + beta p on the window, q = A p, chunk partials of p.q.  Nodes
+    // past the CTA's last carry zeros through (their sums add 0).
 #pragma unroll
     for (int u = 0; u < NI; ++u) {
       const int o = off(u);
-      if (o < L) win[H + o] = first ? w[u] : fma(beta, win[H + o], w[u]);
+      if constexpr (kSpill) {
+        if (o < L) win[H + o] = first ? w[u] : fma(beta, win[H + o], w[u]);
+      } else {
+        p[u] = first ? w[u] : fma(beta, p[u], w[u]);
+        if (o < L) win[H + o] = p[u];
+      }
     }
-    for (int i = threadIdx.x; i < 2 * H; i += blockDim.x) {
+#pragma unroll
+    for (int v = 0; v < NH; ++v) {
+      const int i = v * blockDim.x + threadIdx.x;
+      if (i < 2 * H) {
+        const int slot = i < H ? i : L + i;
+        win[slot] = first ? halo[i] : fma(beta, win[slot], halo[i]);
+      }
+    }
+    for (int i = NH * blockDim.x + threadIdx.x; i < 2 * H; i += blockDim.x) {
       const int slot = i < H ? i : L + i;
       win[slot] = first ? halo[i] : fma(beta, win[slot], halo[i]);
     }
     __syncthreads();
 #pragma unroll
     for (int h = 0; h < NCH; ++h) {
+      double s[4] = {0.0, 0.0, 0.0, 0.0};
+      if (NC > 0 && fast) {
+#pragma unroll
+        for (int c = 0; c < 9; ++c)
+#pragma unroll
+          for (int it = 0; it < 4; ++it) {
+            const int u = 4 * h + it;
+            s[it] = fma(cf[NC == NI ? u : 0][c], win[H + off(u) + (c / 3 - 1) * k.nny + c % 3 - 1], s[it]);
+          }
+      } else if (!kSpill && k.st_tab) {
+#pragma unroll
+        for (int c = 0; c < 9; ++c)
+#pragma unroll
+          for (int it = 0; it < 4; ++it) {
+            const int u = 4 * h + it;
+            s[it] = fma(k.st_tab[c * k.st_cs + max(kind[u], 0) * k.st_rs],
+                        win[H + off(u) + (c / 3 - 1) * k.nny + c % 3 - 1], s[it]);
+          }
+      } else {
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+          const int u = 4 * h + it;
+          if (off(u) < L) s[it] = row_apply_win(k, kind[u], win, H + off(u), wbase);
+        }
+      }
       double acc = 0.0;
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
-        const int u = 4 * h + it, o = off(u);
-        if (o < L) {
-          q[u] = row_apply_win(k, kind[u], win, H + o, wbase);
-          acc = fma(win[H + o], q[u], acc);
+        const int u = 4 * h + it;
+        q[u] = kind[u] < 0 ? 0.0 : s[it];
+        if constexpr (kSpill) {
+          if (off(u) < L) acc = fma(win[H + off(u)], q[u], acc);
+        } else {
+          acc = fma(p[u], q[u], acc);
         }
       }
-      for (int s = 16; s > 0; s >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, s);
+      for (int s2 = 16; s2 > 0; s2 >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, s2);
       if (lane == 0) wsA[h * NG + grp][gw] = acc;
     }
     asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(PIC_RED_THREADS) : "memory");
@@ -1913,7 +2071,7 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
     }
     __syncwarp();
     double pq;
-    if (!(ok = sum_slots<1>(P, P.slotA, tag, k.nb, true, wsTA, &pq))) break;
+    if (!(ok = exchange<1, 0>(P, P.slotA, tag, k.nb, L, wbase, halo, wsTA, &pq))) break;
     if (pq == 0.0) {
       ierr = 3;
       break;
@@ -1924,17 +2082,28 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
 #pragma unroll
     for (int h = 0; h < NCH; ++h) {
       double arr = 0.0, arw = 0.0;
+      bool exact = true;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const int u = 4 * h + it;
+        r[u] = fma(-alpha, q[u], r[u]);
+        if constexpr (!kSpill) w[u] = div_const(r[u], d[u], y[u], exact);
+      }
+      if (kSpill || !exact) {
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+          const int u = 4 * h + it;
+          // 0 and diag 1 on Dirichlet nodes
+          if constexpr (kSpill) w[u] = kind[u] < 0 ? r[u] : r[u] / s_d[off(u)];
+          else w[u] = r[u] / d[u];
+        }
+      }
 #pragma unroll
       for (int it = 0; it < 4; ++it) {
         const int u = 4 * h + it, o = off(u);
-        if (o < L) {
-          r[u] = fma(-alpha, q[u], r[u]);
-          if constexpr (kSpill) w[u] = r[u] / s_d[o];
-          else w[u] = r[u] / d[u];
-          if (o < H || o >= L - H) st_tagged(P.strip + n0 + o, w[u], tag);
-          arr = fma(r[u], r[u], arr);
-          arw = fma(r[u], w[u], arw);
-        }
+        if (o < L && (o < H || o >= L - H)) st_tagged(P.strip + n0 + o, w[u], tag);
+        arr = fma(r[u], r[u], arr);
+        arw = fma(r[u], w[u], arw);
       }
       for (int s = 16; s > 0; s >>= 1) {
         arr = arr + __shfl_xor_sync(0xffffffffu, arr, s);
@@ -1956,30 +2125,23 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
       }
     }
     __syncwarp();
-    // off the path of the reductions: x, and the halo of w
+    // off the path of the reductions: x
 #pragma unroll
     for (int u = 0; u < NI; ++u) {
       const int o = off(u);
       if (o < L) {
         if constexpr (kSpill) s_x[o] = fma(alpha, win[H + o], s_x[o]);
-        else x[u] = fma(alpha, win[H + o], x[u]);
+        else x[u] = fma(alpha, p[u], x[u]);
       }
     }
-    for (int i0 = 0; i0 < 2 * H; i0 += blockDim.x) {
-      const int i = i0 + threadIdx.x;
-      const int64_t m = wbase + (i < H ? i : L + i);
-      const bool want = i < 2 * H && m >= 0 && m < k.nn;
-      double v;
-      ok = ok && poll_tagged<1>(want, P.strip + m, tag, &v, P.bar_err, P.spin_limit);
-      if (want) halo[i] = v;
-    }
     double tot[2];
-    if (!(ok = sum_slots<2>(P, P.slotB, tag, k.nb, ok, wsTB, tot))) break;
+    if (!(ok = exchange<2, NH>(P, P.slotB, tag, k.nb, L, wbase, halo, wsTB, tot))) break;
     normR = tot[0];
     rho0 = rho;
     rho = tot[1];
     ++iter;
-    if (normR / normRHS <= tol2) done = 1;
+    // the division only where the comparison could turn on its rounding
+    if (!(normR > 2.0 * tol2 * normRHS) && normR / normRHS <= tol2) done = 1;
     else if (iter >= maxit) { ierr = 1; done = 1; }
     else if (rho0 == 0.0) { ierr = 2; done = 1; }
     else beta = rho / rho0;
@@ -2397,10 +2559,10 @@ __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a
 
 // A*v for one node in the vector type: FP64 with the FP64 coefficients, FP32
 // with their FP32 copies (same rows, same order).
-template <class V, class F>
+template <class V, int EX, class F>
 __device__ __forceinline__ V row_apply_v(const PcgK &k, int64_t n, F v) {
   if constexpr (sizeof(V) == sizeof(double)) {
-    return row_apply(k, n, v);
+    return row_apply<EX>(k, n, v);
   } else {
     const int kind = k.row_kind[n];
     if (kind < 0) return 0.0f;
@@ -2411,6 +2573,15 @@ __device__ __forceinline__ V row_apply_v(const PcgK &k, int64_t n, F v) {
       for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int c = 0; c < 3; ++c) acc = fmaf(c_stencil32[kind][3 * a + c], v(base + (int64_t)a * k.nny + c), acc);
+    } else if (EX == 1) {
+      const bool edge = n < k.nny + 1 || n >= k.nn - k.nny - 1;
+      float val[9], xv[9];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) val[q] = k.st_tab32[q * k.st_cs + kind * k.st_rs];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) xv[q] = v(stencil_node(k, n, edge, q));
+#pragma unroll
+      for (int q = 0; q < 9; ++q) acc = fmaf(val[q], xv[q], acc);
     } else {
       const int rix = kind - k.n_mat;
       const int cnt = k.ex_cnt[rix];
@@ -2477,7 +2648,7 @@ __device__ __forceinline__ void coarse_gemv(const FcgP<V> &F, int nc, double *s_
   }
 }
 
-template <class V>
+template <class V, int EX>
 __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
   extern __shared__ double fcg_smem[];  // the coarse right-hand side (coarse_gemv)
   const PcgK &k = F.k;
@@ -2534,7 +2705,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
           } else {
             auto z1 = [&](int64_t m) { return (om * rnew(m)) * F.dinv[m]; };
             F.zA[n] = z1(n);
-            F.t[n] = rv - row_apply_v<V>(k, n, z1);
+            F.t[n] = rv - row_apply_v<V, EX>(k, n, z1);
           }
         }
       }
@@ -2676,7 +2847,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
           V zf = (V)0;
           if (k.row_kind[n] >= 0) {
             auto za = [&](int64_t m) { return F.zA[m]; };
-            zf = vfma(om * F.dinv[n], r[n] - row_apply_v<V>(k, n, za), za(n));
+            zf = vfma(om * F.dinv[n], r[n] - row_apply_v<V, EX>(k, n, za), za(n));
           }
           F.zF[n] = zf;
           if (have_old) acc_zq = fma((double)zf, (double)Ql[n], acc_zq);
@@ -2705,7 +2876,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
         const int64_t n = (int64_t)c * kWide + threadIdx.x;
         if (n < nn) {
           const V pv = pnew(n);
-          const V qv = row_apply_v<V>(k, n, pnew);
+          const V qv = row_apply_v<V, EX>(k, n, pnew);
           Pn[n] = pv;
           Qn[n] = qv;
           acc[0] = fma((double)pv, (double)qv, acc[0]);
@@ -2961,7 +3132,7 @@ static void free_all() {
   F(g.d_phi_dir); F(g.d_cell_volume); F(g.d_rhs_fix); F(g.d_mass_q1); F(g.d_ife_mass); F(g.d_mass_rows);
   F(g.d_rf_nodes); F(g.d_rf_base);
   F(g.d_xt_ptr); F(g.d_xt_col); F(g.d_xt_val); F(g.d_row_kind); F(g.d_ex_cnt); F(g.d_ex_col);
-  F(g.d_ex_val); F(g.d_ex_val32); F(g.d_fcg32); F(g.d_diag); F(g.d_ppr_kind); F(g.d_ppr_ptr); F(g.d_ppr_nodes); F(g.d_ppr_rows);
+  F(g.d_ex_val); F(g.d_ex_val32); F(g.d_st_tab); F(g.d_st_tab32); F(g.d_fcg32); F(g.d_diag); F(g.d_ppr_kind); F(g.d_ppr_ptr); F(g.d_ppr_nodes); F(g.d_ppr_rows);
   F(g.d_ppr_h); F(g.d_phi); F(g.d_rho); F(g.d_efx); F(g.d_efy); F(g.d_efxy); F(g.d_coef); F(g.d_coef32); F(g.d_b); F(g.d_x);
   F(g.d_r); F(g.d_w); F(g.d_p[0]); F(g.d_p[1]); F(g.d_q); F(g.d_part); F(g.d_pcg); F(g.d_bar);
   F(g.d_pcg_slot); F(g.d_pcg_strip);
@@ -3220,6 +3391,10 @@ static PcgK pcg_k(int parity) {
   k.ex_col = g.d_ex_col;
   k.ex_val = g.d_ex_val;
   k.ex_val32 = g.d_ex_val32;
+  k.st_tab = g.d_st_tab;
+  k.st_tab32 = g.d_st_tab32;
+  k.st_cs = g.st_cs;
+  k.st_rs = g.st_rs;
   k.diag = g.d_diag;
   k.x = g.d_x;
   k.r = g.d_r;
@@ -3519,6 +3694,12 @@ static int fcg_graph_launch(int i) {
   return PIC_OK;
 }
 
+// the persistent FCG for this context's explicit rows
+template <class V>
+static const void *fcg_fn() {
+  return g.ex_stencil ? (const void *)k_fcg_persist<V, 1> : (const void *)k_fcg_persist<V, 0>;
+}
+
 static int fcg_alloc() {
   if (g.d_fcg_P) return PIC_OK;
   int rc;
@@ -3592,7 +3773,7 @@ static int run_fcg_persist64(pic_solve_stats *stats, int *fcg_iters, int *rc_out
   F.P1 = g.d_fcg_P + nn;
   F.Q0 = g.d_fcg_Q;
   F.Q1 = g.d_fcg_Q + nn;
-  const void *fn = (const void *)k_fcg_persist<double>;
+  const void *fn = fcg_fn<double>();
   const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double);  // coarse_gemv's staging
   if (!g.fcg_smem_set || g.fcg_smem_set != smem) {
     PIC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -3788,7 +3969,7 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
         in.maxit = hs.maxit - total;
         in.stall_window = 50;
         PIC_CUDA(cudaMemcpyAsync(g.d_fcg, &in, sizeof in, cudaMemcpyHostToDevice, g.st));
-        if ((rc = launch(F, (const void *)k_fcg_persist<float>))) { *rc_out = rc; return 1; }
+        if ((rc = launch(F, fcg_fn<float>()))) { *rc_out = rc; return 1; }
         PIC_CUDA(cudaMemcpyAsync(&in, g.d_fcg, sizeof in, cudaMemcpyDeviceToHost, g.st));
         PIC_CUDA(cudaStreamSynchronize(g.st));
         if (in.ierr == 7) {
@@ -3822,7 +4003,7 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
     F.Q0 = g.d_fcg_Q;
     F.Q1 = g.d_fcg_Q + nn;
     for (;;) {
-      if ((rc = launch(F, (const void *)k_fcg_persist<double>))) { *rc_out = rc; return 1; }
+      if ((rc = launch(F, fcg_fn<double>()))) { *rc_out = rc; return 1; }
       PIC_CUDA(cudaMemcpyAsync(&hs, g.d_fcg, sizeof hs, cudaMemcpyDeviceToHost, g.st));
       PIC_CUDA(cudaStreamSynchronize(g.st));
       if (hs.ierr == 7) {
@@ -4333,9 +4514,13 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     };
     std::vector<std::pair<int64_t, double>> ent;
     g.n_mat = 0;
-    // pass 1: stencils from rows whose four elements are one non-interface material
-    for (int i = 1; i < m.nnx - 1 && g.n_mat < 16; ++i)
-      for (int j = 1; j < nny - 1 && g.n_mat < 16; ++j) {
+    // pass 1: stencils from rows whose four elements are one non-interface
+    // material.  They go to constant memory, which serves a warp whose lanes
+    // read one stencil; a mesh with more than fit (r-z: one per radius, so
+    // the lanes of a warp differ) keeps none there.
+    bool many = false;
+    for (int i = 1; i < m.nnx - 1 && !many; ++i)
+      for (int j = 1; j < nny - 1 && !many; ++j) {
         int64_t n = (int64_t)i * nny + j;
         int u = mesh->node_type[n];
         if (u <= 0) continue;
@@ -4357,8 +4542,39 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
         if (!ok) continue;
         bool known = false;
         for (int q = 0; q < g.n_mat && !known; ++q) known = std::memcmp(g.h_stencil[q], S, sizeof S) == 0;
-        if (!known) std::memcpy(g.h_stencil[g.n_mat++], S, sizeof S);
+        if (known) continue;
+        many = g.n_mat == 16;
+        if (!many) std::memcpy(g.h_stencil[g.n_mat++], S, sizeof S);
       }
+    if (many) g.n_mat = 0;
+    // Explicit rows whose entries lie in their 3x3 neighbourhood in column
+    // order (as the mesh builder writes them) are stored as stencils, 0 where
+    // there is no entry, each distinct one once: no column indices, and on
+    // r-z meshes a table of one stencil per radius (72 KB at 1024) in place
+    // of 108 B a node.
+    bool as_stencil = true;
+    // stencil position of column n + d in row n (j: its row of the grid), -1
+    // outside the 3x3 neighbourhood
+    auto position = [&](int64_t d, int j) {
+      const int a = d < -1 ? -1 : d > 1 ? 1 : 0;
+      const int64_t c = d - (int64_t)a * nny;
+      return c < -1 || c > 1 || (c < 0 && j == 0) || (c > 0 && j == nny - 1) ? -1 : 3 * (a + 1) + (int)c + 1;
+    };
+    for (int i = 0; i < m.nnx && as_stencil; ++i)
+      for (int j = 0; j < nny && as_stencil; ++j) {
+        const int64_t n = (int64_t)i * nny + j;
+        const int u = mesh->node_type[n];
+        if (u <= 0) continue;
+        int last = -1;
+        for (int64_t q = mesh->a_srow[u - 1] - 1; q < mesh->a_srow[u] - 1; ++q) {
+          const int at = position(u2n[mesh->a_jcol[q] - 1] - n, j);
+          as_stencil = as_stencil && at > last;
+          last = at;
+        }
+      }
+    g.ex_stencil = as_stencil;
+    std::vector<std::array<double, 9>> st_rows;
+    std::unordered_map<std::string, int32_t> st_index;
     std::vector<int32_t> kind(nn, -1), ex_cnt, ex_col;
     std::vector<double> ex_val, diag(nn, 1.0);
     for (int64_t n = 0; n < nn; ++n) {
@@ -4390,6 +4606,21 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
           set_error("pic_init: stiffness row with more than 9 entries");
           return PIC_ERR_ARG;
         }
+        if (as_stencil) {
+          std::array<double, 9> S;
+          S.fill(0.0);
+          for (auto &pr : ent) S[position(pr.first - n, j)] = pr.second;
+          // the previous column's row at this radius, mostly, on r-z meshes
+          const int32_t before = i > 0 ? kind[n - nny] - g.n_mat : -1;
+          if (before >= 0 && std::memcmp(st_rows[before].data(), S.data(), sizeof S) == 0) {
+            kind[n] = g.n_mat + before;
+            continue;
+          }
+          const auto it = st_index.emplace(std::string((const char *)S.data(), sizeof S), (int32_t)st_rows.size());
+          if (it.second) st_rows.push_back(S);
+          kind[n] = g.n_mat + it.first->second;
+          continue;
+        }
         kind[n] = g.n_mat + (int32_t)ex_cnt.size();
         ex_cnt.push_back((int32_t)ent.size());
         for (auto &pr : ent)
@@ -4408,6 +4639,21 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
       PIC_CUDA(cudaMemcpyToSymbol(c_stencil32, st32, sizeof st32));
       std::vector<float> ev32(ex_val.begin(), ex_val.end());
       if ((rc = upload(&g.d_ex_val32, ev32.data(), ev32.size()))) return rc;
+      if (as_stencil) {  // the material stencils first: a row's kind is its index
+        const int n_tab = g.n_mat + (int)st_rows.size();
+        // Position by position where the lanes of a warp read consecutive
+        // kinds (r-z: one per radius); each stencil in one piece where an
+        // explicit row is alone among regular ones (interface rows)
+        g.st_cs = many ? n_tab : 1;
+        g.st_rs = many ? 1 : 9;
+        std::vector<double> t((size_t)9 * n_tab);
+        for (int r = 0; r < n_tab; ++r)
+          for (int q = 0; q < 9; ++q)
+            t[(size_t)q * g.st_cs + (size_t)r * g.st_rs] = r < g.n_mat ? g.h_stencil[r][q] : st_rows[r - g.n_mat][q];
+        const std::vector<float> t32(t.begin(), t.end());
+        if ((rc = upload(&g.d_st_tab, t.data(), t.size()))) return rc;
+        if ((rc = upload(&g.d_st_tab32, t32.data(), t32.size()))) return rc;
+      }
     }
     if ((rc = upload(&g.d_row_kind, kind.data(), kind.size()))) return rc;
     if ((rc = upload(&g.d_ex_cnt, ex_cnt.data(), ex_cnt.size()))) return rc;
@@ -4601,8 +4847,8 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     g.coop_grid = (want && coop && per_sm > 0) ? std::min(g.red_blocks, per_sm * nsm) : 0;
     int per_sm_f = 0;
     int per_sm_f32 = 0;
-    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, k_fcg_persist<double>, kWide, 0));
-    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f32, k_fcg_persist<float>, kWide, 0));
+    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, fcg_fn<double>(), kWide, 0));
+    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f32, fcg_fn<float>(), kWide, 0));
     per_sm_f = std::min(per_sm_f, per_sm_f32);
     const char *envf = getenv("PIC_FCG_PERSISTENT");
     const bool want_f = !(envf && envf[0] == '0');
