@@ -336,7 +336,8 @@ __global__ void k_adam(int64_t n, float *__restrict__ p, const float *__restrict
   if (pb) pb[i] = __float2bfloat16(pi);
 }
 
-// Weight gradient of a 3x3 'same' convolution on the CUDA cores.  CTA =
+// Weight gradient of a 3x3 'same' convolution on the CUDA cores, for channel
+// counts that are no multiple of 8.  CTA =
 // (32 output channels x 32 input channels) x a strided set of 32-pixel tiles;
 // each thread accumulates 9 taps x 4 input channels of one output channel in
 // registers, from tiles of dy and of the 9 shifted x staged in shared memory.
@@ -394,6 +395,151 @@ __global__ void __launch_bounds__(256) k_wgrad(int n, int h, int w, int c, int k
       const int cx = cb * 32 + cq + q;
       if (cx < c && acc[tap][q] != 0.0f) atomicAdd(dw + ((int64_t)kx * 9 + tap) * c + cx, acc[tap][q]);
     }
+}
+
+// The same on the tensor cores, for channel counts that are multiples of 8
+// (16-byte rows): dW = sum over pixels of dy^T x, a GEMM whose K is the pixels.
+// CTA = (16 MT output channels x 32 input channels) x a strided set of tiles
+// of 4 image rows x 32 pixels.  The tile's dy and its x with a one-pixel rim
+// are staged once (cp.async, two stages, zeros outside the image) and serve
+// all nine taps: warp t owns tap t and reads x at its shift.  Pixels run along
+// the rows of both operands in shared memory, so both are read transposed
+// (ldmatrix.trans); rows are padded by 16 bytes, which spreads the eight rows
+// of a matrix over all banks.  BF16 products, FP32 accumulation; partial sums
+// of the CTAs meet in dw by atomicAdd as before.
+// mma.sync and not tcgen05: the widest layer needs 2.8 GMAC a call (a few
+// microseconds at either rate) and the call is bound by staging and latency;
+// M is 32..64, half the smallest full-rate tcgen05 tile.
+// At 4 x 128^2: 306 -> 12 us a call (mean over the network's ten layers).
+constexpr int WG_ROWS = 4, WG_PIX = 32, WG_THREADS = 9 * 32;
+constexpr int WG_XS = 40;  // x row in shared memory: 32 channels + 8 of padding
+
+template <int MT>
+struct WgTile {
+  static constexpr int DS = 16 * MT + 8;
+  bf16 x[(WG_ROWS + 2) * (WG_PIX + 2)][WG_XS];
+  bf16 dy[WG_ROWS * WG_PIX][DS];
+};
+
+__device__ __forceinline__ void wg_cp16(bf16 *dst, const bf16 *src, bool valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int bytes = valid ? 16 : 0;  // 0: the 16 bytes are zero-filled, src is not read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void wg_ldsm4t(unsigned (&r)[4], const bf16 *p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+
+__device__ __forceinline__ void wg_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+               "{%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <int MT>
+__device__ __forceinline__ void wg_stage(WgTile<MT> &T, int tile, int ti, int tj, int h, int w, int c, int k, int kb,
+                                         int cb, const bf16 *__restrict__ x, const bf16 *__restrict__ dy) {
+  const int b = tile / (ti * tj), i0 = tile / tj % ti * WG_ROWS, j0 = tile % tj * WG_PIX;
+  for (int e = threadIdx.x; e < (WG_ROWS + 2) * (WG_PIX + 2) * 4; e += WG_THREADS) {
+    const int g = e & 3, px = e >> 2;
+    const int i = i0 + px / (WG_PIX + 2) - 1, j = j0 + px % (WG_PIX + 2) - 1, ch = cb * 32 + 8 * g;
+    const bool in = i >= 0 && i < h && j >= 0 && j < w && ch < c;
+    wg_cp16(&T.x[px][8 * g], in ? x + (((int64_t)b * h + i) * w + j) * c + ch : x, in);
+  }
+  for (int e = threadIdx.x; e < WG_ROWS * WG_PIX * 2 * MT; e += WG_THREADS) {
+    const int g = e % (2 * MT), px = e / (2 * MT);
+    const int i = i0 + px / WG_PIX, j = j0 + px % WG_PIX, ch = kb * 16 * MT + 8 * g;
+    const bool in = i < h && j < w && ch < k;
+    wg_cp16(&T.dy[px][8 * g], in ? dy + (((int64_t)b * h + i) * w + j) * k + ch : dy, in);
+  }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int MT>
+__global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, int c, int k, const bf16 *__restrict__ x,
+                                                          const bf16 *__restrict__ dy, float *__restrict__ dw) {
+  extern __shared__ __align__(128) unsigned char wg_smem[];
+  WgTile<MT> *T = reinterpret_cast<WgTile<MT> *>(wg_smem);
+  const int ncb = (c + 31) / 32, kb = blockIdx.x / ncb, cb = blockIdx.x % ncb;
+  const int ti = (h + WG_ROWS - 1) / WG_ROWS, tj = (w + WG_PIX - 1) / WG_PIX, tiles = n * ti * tj;
+  const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5, tr = tap / 3, ts = tap % 3;
+  float acc[MT][4][4];
+#pragma unroll
+  for (int a = 0; a < MT; ++a)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[a][q][e] = 0.0f;
+  const int apix = (lane & 7) + ((lane >> 4) & 1) * 8, ach = ((lane >> 3) & 1) * 8;
+  const int bpix = (lane & 7) + ((lane >> 3) & 1) * 8, bch = ((lane >> 4) & 1) * 8;
+  int stage = 0;
+  if ((int)blockIdx.y < tiles) wg_stage<MT>(T[0], blockIdx.y, ti, tj, h, w, c, k, kb, cb, x, dy);
+  for (int tile = blockIdx.y; tile < tiles; tile += gridDim.y, stage ^= 1) {
+    const int next = tile + gridDim.y;
+    if (next < tiles) {
+      wg_stage<MT>(T[stage ^ 1], next, ti, tj, h, w, c, k, kb, cb, x, dy);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const WgTile<MT> &S = T[stage];
+    for (int row = 0; row < WG_ROWS; ++row) {
+      unsigned A[2][MT][4], B[2][2][4];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {  // 16 pixels of the row each
+#pragma unroll
+        for (int a = 0; a < MT; ++a) wg_ldsm4t(A[s][a], &S.dy[row * WG_PIX + 16 * s + apix][16 * a + ach]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          wg_ldsm4t(B[s][q], &S.x[(row + tr) * (WG_PIX + 2) + 16 * s + ts + bpix][16 * q + bch]);
+      }
+#pragma unroll
+      for (int a = 0; a < MT; ++a)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          // the row's sum from zero, then a rounded add: the tensor cores
+          // truncate what they add to, so a long chain in them drifts
+          float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+          for (int s = 0; s < 2; ++s) wg_mma(t, A[s][a], B[s][q >> 1][2 * (q & 1)], B[s][q >> 1][2 * (q & 1) + 1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[a][q][e] += t[e];
+        }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int a = 0; a < MT; ++a)
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int kx = kb * 16 * MT + 16 * a + (lane >> 2) + 8 * (e >> 1);
+        const int cx = cb * 32 + 8 * q + 2 * (lane & 3) + (e & 1);
+        if (kx < k && cx < c && acc[a][q][e] != 0.0f) atomicAdd(dw + ((int64_t)kx * 9 + tap) * c + cx, acc[a][q][e]);
+      }
+}
+
+// Grid: the CTAs of a (k, c) block share its tiles; two CTAs per SM in all,
+// each CTA taking at least two tiles while there are enough (fewer atomics).
+template <int MT>
+int run_wgrad_mma(int n, int h, int w, int c, int k, const bf16 *x, const bf16 *dy, float *dw, cudaStream_t st) {
+  const size_t smem = 2 * sizeof(WgTile<MT>);
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(k_wgrad_mma<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return UNET_ERR_CUDA;
+  const unsigned gx = (unsigned)(((k + 16 * MT - 1) / (16 * MT)) * ((c + 31) / 32));
+  const int64_t tiles = (int64_t)n * ((h + WG_ROWS - 1) / WG_ROWS) * ((w + WG_PIX - 1) / WG_PIX);
+  int64_t gy = (2 * 148 + gx - 1) / gx;
+  if (gy > (tiles + 1) / 2) gy = (tiles + 1) / 2;
+  k_wgrad_mma<MT><<<dim3(gx, (unsigned)gy), WG_THREADS, smem, st>>>(n, h, w, c, k, x, dy, dw);
+  return launched();
 }
 
 __global__ void k_fill(int64_t n, float *p, float v) {
@@ -513,6 +659,12 @@ int unet_wgrad(int32_t n, int32_t h, int32_t w, int32_t c, int32_t k, const void
                void *stream) {
   if (n < 1 || h < 1 || w < 1 || c < 1 || k < 1) return UNET_ERR_SHAPE;
   const int64_t np = (int64_t)n * h * w;
+  // the tensor-core form wants 16-byte channel groups (and indexes tiles in
+  // 32 bits); other shapes and alignments take the CUDA cores
+  if (c % 8 == 0 && k % 8 == 0 && (((uintptr_t)x | (uintptr_t)dy) & 15) == 0 && np < ((int64_t)1 << 31)) {
+    if (k > 32) return run_wgrad_mma<4>(n, h, w, c, k, (const bf16 *)x, (const bf16 *)dy, dw, (cudaStream_t)stream);
+    return run_wgrad_mma<2>(n, h, w, c, k, (const bf16 *)x, (const bf16 *)dy, dw, (cudaStream_t)stream);
+  }
   const unsigned gx = (unsigned)(((k + 31) / 32) * ((c + 31) / 32));
   unsigned gy = (unsigned)((np + 31) / 32);
   const unsigned cap = (148u * 8u + gx - 1) / gx;

@@ -473,3 +473,26 @@ def test_persistent_fcg_matches_graph_path():
             sim.close()
     assert abs(out[0][0] - out[1][0]) <= 2
     assert np.abs(out[0][1] - out[1][1]).max() <= 1e-7 * np.abs(out[0][1]).max()
+
+
+# the tiles of the tensor-core weight gradient are 4 rows x 32 pixels x 32
+# input channels x 32 or 64 output channels: edges and remainders of each, the
+# network's widest layer, and channel counts left to the CUDA cores.  FP32
+# sums of up to 6e3 exact products: 1e-5 of the result's norm as above.
+@gpu
+@pytest.mark.parametrize("n,c,k,h,w", [(1, 8, 8, 1, 1), (1, 8, 32, 3, 31), (2, 32, 32, 4, 32), (3, 40, 24, 5, 33),
+                                       (1, 192, 64, 64, 64), (2, 64, 72, 9, 65), (1, 33, 20, 6, 7), (1, 5, 40, 8, 40)])
+def test_wgrad_tiles_match_fp64(n, c, k, h, w):
+    from pic_b200 import unet
+    import torch.nn.functional as F
+    lib = unet.load()
+    g = torch.Generator().manual_seed(11 * c + k)
+    x = _bf(torch.randn(n, h, w, c, generator=g))
+    dy = _bf(torch.randn(n, h, w, k, generator=g))
+    wt = torch.zeros(k, c, 3, 3, dtype=torch.float64, requires_grad=True)
+    F.conv2d(x.double().permute(0, 3, 1, 2), wt, padding=1).backward(dy.double().permute(0, 3, 1, 2))
+    dw = torch.ones(k, 3, 3, c, dtype=torch.float32, device="cuda")  # accumulated into
+    xd, dyd = x.cuda(), dy.cuda()
+    assert lib.unet_wgrad(n, h, w, c, k, P(xd), P(dyd), P(dw), None) == 0
+    torch.cuda.synchronize()
+    assert _rel(dw.double().cpu() - 1.0, wt.grad.permute(0, 2, 3, 1)) < 1e-5
