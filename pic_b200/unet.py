@@ -101,6 +101,38 @@ class DeviceArray:
                                          "version": 3, "strides": None}
 
 
+class ParamSet(dict):
+    """Parameters by name, each {"p", "bf", "g", "m", "v"} views into one buffer
+    a kind (`flat`), so that clearing the gradients and Adam are one launch
+    each and not one a parameter.  Every parameter starts on a multiple of
+    ALIGN elements (the tensor cores' loads want 16-byte rows); the elements
+    between are zero and stay zero."""
+
+    ALIGN = 128
+
+    def __init__(self, torch, values: dict):
+        super().__init__()
+        at, total = {}, 0
+        for name, t in values.items():
+            at[name] = total
+            total += -(-t.numel() // self.ALIGN) * self.ALIGN
+        new = lambda dtype: torch.zeros(total, dtype=dtype, device="cuda")  # noqa: E731
+        self.flat = {k: new(torch.bfloat16 if k == "bf" else torch.float32) for k in ("p", "bf", "g", "m", "v")}
+        for name, t in values.items():
+            part = slice(at[name], at[name] + t.numel())
+            self[name] = {k: f[part].view(t.shape) for k, f in self.flat.items()}
+            self[name]["p"].copy_(t)
+            self[name]["bf"].copy_(self[name]["p"].to(torch.bfloat16))
+        self.places = self._places()
+
+    def _places(self) -> list:
+        return [(v[k].data_ptr(), v[k].numel()) for v in self.values() for k in ("p", "bf", "g", "m", "v")]
+
+    def one_buffer(self) -> bool:
+        """Whether every parameter still is its view (none was replaced)."""
+        return self._places() == self.places
+
+
 class UNet:
     """Parameters (FP32 masters + BF16 copies), activations, forward,
     backward and Adam, all through libpicunet.so."""
@@ -111,22 +143,24 @@ class UNet:
         self.lib = load()
         self.stream = stream
         g = torch.Generator().manual_seed(seed)
-        self.params = {}
+        values = {}
         for name, cin, cout in LAYERS:
-            w = torch.randn(cout, 3, 3, cin, generator=g) * math.sqrt(2.0 / (9 * cin))
-            self._add(name + ".w", w)
-            self._add(name + ".b", torch.zeros(cout))
-        self._add("head.w", torch.randn(32, generator=g) * math.sqrt(1.0 / 32))
-        self._add("head.b", torch.zeros(1))
+            values[name + ".w"] = torch.randn(cout, 3, 3, cin, generator=g) * math.sqrt(2.0 / (9 * cin))
+            values[name + ".b"] = torch.zeros(cout)
+        values["head.w"] = torch.randn(32, generator=g) * math.sqrt(1.0 / 32)
+        values["head.b"] = torch.zeros(1)
+        self.params = ParamSet(torch, values)
         self.t = 0
         self.shape = None
         self.ws = None
 
-    def _add(self, name, t32):
-        torch = self.torch
-        p = t32.to("cuda", torch.float32).contiguous()
-        self.params[name] = {"p": p, "bf": p.to(torch.bfloat16).contiguous(), "g": torch.zeros_like(p),
-                             "m": torch.zeros_like(p), "v": torch.zeros_like(p)}
+    def _buffers(self):
+        """What the element-wise kernels run over: the parameters' common
+        buffers, or each parameter where some were replaced."""
+        P = self.params
+        if isinstance(P, ParamSet) and P.one_buffer():
+            return [P.flat]
+        return list(P.values())
 
     def state(self) -> dict:
         return {k: v["p"].detach().cpu().clone() for k, v in self.params.items()}
@@ -217,7 +251,7 @@ class UNet:
                             _p(self.ga[inp]), None, _p(self.ws), self.ws.numel(), None, st), "dgrad " + name)
 
     def zero_grad(self):
-        for v in self.params.values():
+        for v in self._buffers():
             _ck(self.lib.unet_fill_f32(v["g"].numel(), _p(v["g"]), 0.0, self.stream), "zero")
 
     def backward(self):
@@ -247,7 +281,7 @@ class UNet:
 
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
         self.t += 1
-        for v in self.params.values():
+        for v in self._buffers():
             _ck(self.lib.unet_adam(v["p"].numel(), _p(v["p"]), _p(v["g"]), _p(v["m"]), _p(v["v"]), _p(v["bf"]),
                                    lr, b1, b2, eps, self.t, self.stream), "adam")
 

@@ -496,3 +496,30 @@ def test_wgrad_tiles_match_fp64(n, c, k, h, w):
     assert lib.unet_wgrad(n, h, w, c, k, P(xd), P(dyd), P(dw), None) == 0
     torch.cuda.synchronize()
     assert _rel(dw.double().cpu() - 1.0, wt.grad.permute(0, 2, 3, 1)) < 1e-5
+
+
+@gpu
+def test_params_in_one_buffer_and_replaced_ones_take_the_same_step():
+    """Clearing and Adam over the common buffers, and one parameter at a time
+    when one was replaced: the same weights, and nothing between them moves."""
+    from pic_b200 import unet
+    nets = [unet.UNet(seed=5), unet.UNet(seed=5)]
+    for k in ("p", "bf", "g", "m", "v"):  # the second net's b.w leaves the buffer
+        nets[1].params["ba.w"][k] = nets[1].params["ba.w"][k].clone()
+    assert nets[0].params.one_buffer() and not nets[1].params.one_buffer()
+    for step in range(3):
+        g = torch.Generator().manual_seed(step)
+        grads = {k: torch.randn(v["p"].shape, generator=g) for k, v in nets[0].params.items()}
+        for net in nets:
+            net.zero_grad()
+            assert all(not v["g"].any() for v in net.params.values())
+            for k, v in net.params.items():
+                v["g"].copy_(grads[k])
+            net.adam(1e-2)
+    torch.cuda.synchronize()
+    for k, v in nets[0].params.items():
+        for kind in ("p", "bf", "m", "v"):
+            assert torch.equal(v[kind], nets[1].params[k][kind]), (k, kind)
+        assert v["p"].data_ptr() % 16 == 0 and v["bf"].data_ptr() % 16 == 0
+    used = sum(v["p"].numel() for v in nets[0].params.values())
+    assert int((nets[0].params.flat["p"] != 0).sum()) <= used
