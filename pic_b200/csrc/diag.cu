@@ -19,6 +19,7 @@
 // position rebuilt from a mixed-precision particle equals the one the
 // download path writes.
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "pic_ctx.h"
@@ -38,43 +39,69 @@ struct ProfK {
 };
 
 // Output_To_Tecplot_IJK_2D.f90:184-215: a column's nodes in node order,
-// summed, divided by their count, then scaled for the file (:220-223).
-__global__ void k_average_x(ProfK k) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, c = blockIdx.y;
-  if (i >= k.nnx || c >= k.ncols) return;
-  double v;
-  if (!k.f[c]) {
-    v = k.xs[i] * k.scale[c];
-  } else {
-    const double *col = k.f[c] + (size_t)i * k.nny;
-    double s = 0.0;
-#pragma unroll 8
-    for (int j = 0; j < k.nny; ++j) s = s + col[j];
-    v = (s / (double)k.nny) * k.scale[c];
+// summed, divided by their count, then scaled for the file (:220-223).  The
+// sum of a column is one chain (the reference's order), so a thread takes a
+// column; its nodes are contiguous, so the block loads tiles of 32 columns x
+// 32 nodes with whole lines and the chains read them from shared memory, the
+// next tile's loads in flight behind them (a thread a column straight from
+// memory touched 32 lines a load: 25 -> 8 us at 257 x 257, nine quantities).
+constexpr int kAvgCols = 32, kAvgRows = 32, kAvgThreads = 256;
+
+__global__ void __launch_bounds__(kAvgThreads) k_average_x(ProfK k) {
+  __shared__ double tile[2][kAvgCols][kAvgRows + 1];
+  const int c = blockIdx.y, i0 = blockIdx.x * kAvgCols;
+  const int j = threadIdx.x % kAvgRows, w = threadIdx.x / kAvgRows;  // w: 8 columns apart by kAvgThreads / 32
+  constexpr int NL = kAvgCols * kAvgRows / kAvgThreads;
+  double s = 0.0;
+  if (k.f[c]) {
+    double v[NL];
+    auto load = [&](int j0) {
+#pragma unroll
+      for (int q = 0; q < NL; ++q) {
+        const int i = i0 + w + q * (kAvgThreads / kAvgRows);
+        v[q] = i < k.nnx && j0 + j < k.nny ? k.f[c][(size_t)i * k.nny + j0 + j] : 0.0;
+      }
+    };
+    load(0);
+    int buf = 0;
+    for (int j0 = 0; j0 < k.nny; j0 += kAvgRows, buf ^= 1) {
+#pragma unroll
+      for (int q = 0; q < NL; ++q) tile[buf][w + q * (kAvgThreads / kAvgRows)][j] = v[q];
+      __syncthreads();
+      if (j0 + kAvgRows < k.nny) load(j0 + kAvgRows);
+      if (threadIdx.x < kAvgCols) {
+        const int m = min(kAvgRows, k.nny - j0);
+        for (int q = 0; q < m; ++q) s = s + tile[buf][threadIdx.x][q];
+      }
+    }
   }
-  k.out[(size_t)c * k.nnx + i] = v;
+  const int i = i0 + threadIdx.x;
+  if (threadIdx.x >= kAvgCols || i >= k.nnx) return;
+  k.out[(size_t)c * k.nnx + i] = k.f[c] ? (s / (double)k.nny) * k.scale[c] : k.xs[i] * k.scale[c];
 }
 
 // One species' particle arrays; FP32 data in the first half of the double
-// storage when f32 (x, y then hold the offsets inside the element loc).
+// storage for F32 kernels (x, y then hold the offsets inside the element loc).
 struct PartK {
   const double *x, *vx, *vy, *vz;
   const int32_t *loc;
   int64_t n;
-  int f32;
   int ney;
   double xmin, hx;
 };
 
-__device__ __forceinline__ double vget(const double *a, int f32, int64_t p) {
-  return f32 ? (double)reinterpret_cast<const float *>(a)[p] : a[p];
+template <bool F32>
+__device__ __forceinline__ double vget(const double *a, int64_t p) {
+  if constexpr (F32) return (double)reinterpret_cast<const float *>(a)[p];
+  else return a[p];
 }
 
 // absolute x of a live particle, as the download path writes it
+template <bool F32>
 __device__ __forceinline__ double xget(const PartK &s, int64_t p, int e) {
-  if (!s.f32) return s.x[p];
-  const int i = e / s.ney;
-  return s.xmin + ((double)i + (double)reinterpret_cast<const float *>(s.x)[p]) * s.hx;
+  const double x = vget<F32>(s.x, p);
+  if constexpr (!F32) return x;
+  return s.xmin + ((double)(e / s.ney) + x) * s.hx;
 }
 
 // reference bin edges, evaluated in the reference's order
@@ -95,12 +122,25 @@ __device__ __forceinline__ int find_bin(double v, double t, const double *edge, 
   return -1;
 }
 
-// add 1 to sh[bin] for every lane with bin >= 0, one shared atomic per
-// distinct bin in the warp; all 32 lanes call it
+// The bin of a value at t bin widths from edge[0] where t decides it: off
+// every edge by far more than the few ulps t and the edges are good to (edges
+// within 4096 bins: 1e-12 widths).  -1: outside; -2: too near an edge.
+__device__ __forceinline__ int clear_bin(double t, int n) {
+  if (!(t > -2.0) || !(t < n + 2.0)) return t == t ? -1 : -2;
+  const double f = floor(t);
+  if (t - f < 1e-6 || t - f > 1.0 - 1e-6) return -2;
+  return f >= 0.0 && f < (double)n ? (int)f : -1;
+}
+
+// add 1 to sh[bin] for every lane with bin >= 0; all 32 lanes call it.  The
+// lanes that share lane 0's bin (most of them in a narrow distribution, ions
+// in electron bins) count as one; the others add their own.
 __device__ __forceinline__ void warp_count(unsigned int *sh, int bin) {
-  const unsigned same = __match_any_sync(0xffffffffu, bin);
-  const int lane = threadIdx.x & 31;
-  if (bin >= 0 && lane == __ffs(same) - 1) atomicAdd(&sh[bin], (unsigned)__popc(same));
+  const int b0 = __shfl_sync(0xffffffffu, bin, 0);
+  const unsigned same = __ballot_sync(0xffffffffu, bin == b0);
+  if (bin < 0) return;
+  if (bin != b0) atomicAdd(&sh[bin], 1u);
+  else if ((threadIdx.x & 31) == 0) atomicAdd(&sh[bin], (unsigned)__popc(same));
 }
 
 struct SpecK {
@@ -108,12 +148,18 @@ struct SpecK {
   int nbins;
   double mass, vref, e_max, v_max;
   double e_inv, v_inv;  // nbins / e_max, nbins / v_max
+  double ej_inv;        // nbins / (e_max J_to_eV); NaN (no bin is clear) where that could underflow
   unsigned long long *ce, *cv;
 };
 
 // Output_Energy.f90:55-71 for one species.  The grid-stride loop runs the
 // same number of iterations on every lane of a warp (the base index is
-// uniform), so the whole-warp match is legal.
+// uniform), so the whole-warp votes are legal.  HBM-bound in aim (28 B a
+// particle FP64); 80 -> 42 us for 5.7M FP64 particles against a division, two
+// edge searches and two whole-warp matches a particle.
+constexpr int kSpecBatch = 4;  // particles a lane has in flight
+
+template <bool F32>
 __global__ void __launch_bounds__(256) k_spectrum(SpecK k) {
   extern __shared__ double edges[];  // [nbins+1] energy, [nbins+1] vx edges, then [2][nbins] counts
   double *ee = edges, *ve = edges + k.nbins + 1;
@@ -125,18 +171,41 @@ __global__ void __launch_bounds__(256) k_spectrum(SpecK k) {
   for (int b = threadIdx.x; b < 2 * k.nbins; b += blockDim.x) sh[b] = 0u;
   __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < k.s.n; base += stride) {
-    const int64_t p = base + threadIdx.x;
-    int be = -1, bv = -1;
-    if (p < k.s.n && k.s.loc[p] >= 0) {
-      const double vx = vget(k.s.vx, k.s.f32, p), vy = vget(k.s.vy, k.s.f32, p), vz = vget(k.s.vz, k.s.f32, p);
-      // ParticleOne.f90:235-244 EnergyParticleOne with VFactor, then / JtoeV
-      const double e = ((((0.5 * k.mass) * ((vx * vx + vy * vy) + vz * vz)) * k.vref) * k.vref) / PIC_JTOEV;
-      be = find_bin(e, e * k.e_inv, ee, k.nbins);
-      bv = find_bin(vx, vx * k.v_inv + 0.5 * k.nbins, ve, k.nbins);
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < k.s.n; base += kSpecBatch * stride) {
+    double v[kSpecBatch][3];
+    int e[kSpecBatch];
+#pragma unroll
+    for (int u = 0; u < kSpecBatch; ++u) {
+      const int64_t p = base + u * stride + threadIdx.x;
+      e[u] = -1;
+      v[u][0] = v[u][1] = v[u][2] = 0.0;
+      if (p < k.s.n) {
+        e[u] = k.s.loc[p];
+        v[u][0] = vget<F32>(k.s.vx, p);
+        v[u][1] = vget<F32>(k.s.vy, p);
+        v[u][2] = vget<F32>(k.s.vz, p);
+      }
     }
-    warp_count(sh, be);
-    warp_count(sh + k.nbins, bv);
+#pragma unroll
+    for (int u = 0; u < kSpecBatch; ++u) {
+      int be = -1, bv = -1;
+      if (e[u] >= 0) {
+        const double vx = v[u][0], vy = v[u][1], vz = v[u][2];
+        // ParticleOne.f90:235-244 EnergyParticleOne with VFactor, then / JtoeV;
+        // the division and the edges only where they can decide the bin
+        const double ej = (((0.5 * k.mass) * ((vx * vx + vy * vy) + vz * vz)) * k.vref) * k.vref;
+        const double tv = vx * k.v_inv + 0.5 * k.nbins;
+        be = clear_bin(ej * k.ej_inv, k.nbins);
+        if (be == -2) {
+          const double ev = ej / PIC_JTOEV;
+          be = find_bin(ev, ev * k.e_inv, ee, k.nbins);
+        }
+        bv = clear_bin(tv, k.nbins);
+        if (bv == -2) bv = find_bin(vx, tv, ve, k.nbins);
+      }
+      warp_count(sh, be);
+      warp_count(sh + k.nbins, bv);
+    }
   }
   __syncthreads();
   for (int b = threadIdx.x; b < k.nbins; b += blockDim.x) {
@@ -162,9 +231,20 @@ __device__ __forceinline__ int x_bin(double X, int nbins) {
 }
 
 // pass 1 (OUTPUT_velocity.f90:55-63): count and velocity sums per column;
-// pass 2 (:80-87, kSecond): sums of (v - drift)^2
-template <bool kSecond>
-__global__ void __launch_bounds__(256) k_vmoments(MomK k) {
+// pass 2 (:80-87, kSecond): sums of (v - drift)^2.
+//
+// Every warp takes one contiguous run of particles.  They are sorted by cell,
+// so a run stays within one x column, or two neighbours where a column's edge
+// (one Debye length, about one cell) crosses the cells, for a long time: the
+// lanes sum those two columns (base, base + 1) in registers and the warp adds
+// them to the CTA's shared sums only when a particle leaves them.  Lanes
+// outside the two (unsorted particles) add their own.  HBM-bound in aim (36 B
+// a particle FP64); 104 -> 53 us (pass 1) and 112 -> 63 us (pass 2) for 5.7M
+// particles against shuffled warp sums of every 32 particles.
+constexpr int kMomBatch = 2;  // particles a lane has in flight
+
+template <bool kSecond, bool F32>
+__global__ void __launch_bounds__(256, 4) k_vmoments(MomK k) {
   extern __shared__ double shd[];  // [3][nbins] sums, then [3][nbins] drift (pass 2) or [nbins] counts
   double *acc = shd;
   double *dr = shd + 3 * k.nbins;
@@ -176,57 +256,96 @@ __global__ void __launch_bounds__(256) k_vmoments(MomK k) {
   if (!kSecond)
     for (int b = threadIdx.x; b < k.nbins; b += blockDim.x) cnt[b] = 0u;
   __syncthreads();
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < k.s.n; base += stride) {
-    const int64_t p = base + threadIdx.x;
-    int b = -1;
-    double v[3] = {0.0, 0.0, 0.0};
-    if (p < k.s.n) {
-      const int e = k.s.loc[p];
-      if (e >= 0) {
-        b = x_bin(xget(k.s, p, e), k.nbins);
-        v[0] = vget(k.s.vx, k.s.f32, p);
-        v[1] = vget(k.s.vy, k.s.f32, p);
-        v[2] = vget(k.s.vz, k.s.f32, p);
-      }
-    }
-    if (!kSecond) warp_count(cnt, b);
-    double t[3];
-    for (int c = 0; c < 3; ++c) {
-      t[c] = v[c];
-      if (kSecond && b >= 0) {
-        const double d = v[c] - dr[c * k.nbins + b];
-        t[c] = d * d;
-      }
-    }
-    // particles sorted by cell: a warp's particles fall in one x column, or
-    // in two when a column edge (one Debye length, about one cell) crosses
-    // their cells.  Then the warp sums per column first and adds once per
-    // column and component; otherwise every lane adds its own.  Every lane
-    // takes part in each ballot and shuffle (none is skipped by
-    // short-circuiting).
-    const unsigned full = 0xffffffffu;
-    const int b0 = __shfl_sync(full, b, 0);
-    const unsigned m0 = __ballot_sync(full, b == b0);
-    const int src1 = (m0 == full) ? 0 : __ffs(~m0) - 1;
-    const int b1 = __shfl_sync(full, b, src1);
-    const unsigned m1 = __ballot_sync(full, b == b1);
-    if ((m0 | m1) == full) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
+  const int64_t w = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  const int64_t run = ((k.s.n + warps - 1) / warps + 32 * kMomBatch - 1) / (32 * kMomBatch) * (32 * kMomBatch);
+  const int64_t p1 = min(k.s.n, (w + 1) * run);
+  int base = -2;
+  double s0[3] = {0.0, 0.0, 0.0}, s1[3] = {0.0, 0.0, 0.0}, d0[3], d1[3];
+  unsigned c0 = 0, c1 = 0;
+  auto rebase = [&](int b) {  // every lane of the warp, the same b
+    if (base >= 0) {
+#pragma unroll
       for (int c = 0; c < 3; ++c) {
-        double s0 = (b == b0) ? t[c] : 0.0, s1 = (b == b1 && b1 != b0) ? t[c] : 0.0;
         for (int o = 16; o > 0; o >>= 1) {
-          s0 += __shfl_xor_sync(full, s0, o);
-          s1 += __shfl_xor_sync(full, s1, o);
+          s0[c] += __shfl_xor_sync(full, s0[c], o);
+          s1[c] += __shfl_xor_sync(full, s1[c], o);
         }
-        if ((threadIdx.x & 31) == 0) {
-          if (b0 >= 0) atomicAdd(&acc[c * k.nbins + b0], s0);
-          if (b1 != b0 && b1 >= 0) atomicAdd(&acc[c * k.nbins + b1], s1);
+        if (lane == 0) {
+          atomicAdd(&acc[c * k.nbins + base], s0[c]);
+          if (base + 1 < k.nbins) atomicAdd(&acc[c * k.nbins + base + 1], s1[c]);
         }
+        s0[c] = s1[c] = 0.0;
       }
-    } else if (b >= 0) {
-      for (int c = 0; c < 3; ++c) atomicAdd(&acc[c * k.nbins + b], t[c]);
+      if (!kSecond) {
+        c0 = __reduce_add_sync(full, c0);
+        c1 = __reduce_add_sync(full, c1);
+        if (lane == 0) {
+          atomicAdd(&cnt[base], c0);
+          if (base + 1 < k.nbins) atomicAdd(&cnt[base + 1], c1);
+        }
+        c0 = c1 = 0;
+      }
+    }
+    base = b;
+    if (kSecond && b >= 0)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        d0[c] = dr[c * k.nbins + b];
+        d1[c] = b + 1 < k.nbins ? dr[c * k.nbins + b + 1] : 0.0;
+      }
+  };
+  for (int64_t q = w * run; q < p1; q += 32 * kMomBatch) {
+    int b[kMomBatch];
+    double v[kMomBatch][3];
+#pragma unroll
+    for (int u = 0; u < kMomBatch; ++u) {
+      const int64_t p = q + 32 * u + lane;
+      b[u] = -1;
+      v[u][0] = v[u][1] = v[u][2] = 0.0;
+      if (p < p1) {
+        const int e = k.s.loc[p];
+        const double X = xget<F32>(k.s, p, max(e, 0));
+        v[u][0] = vget<F32>(k.s.vx, p);
+        v[u][1] = vget<F32>(k.s.vy, p);
+        v[u][2] = vget<F32>(k.s.vz, p);
+        if (e >= 0) b[u] = x_bin(X, k.nbins);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kMomBatch; ++u) {
+      if (__any_sync(full, b[u] >= 0 && b[u] != base && b[u] != base + 1)) {
+        // the lowest column of this batch (0xffffffff: no live particle)
+        const unsigned lo = __reduce_min_sync(full, b[u] >= 0 ? (unsigned)b[u] : 0xffffffffu);
+        rebase((int)lo);
+      }
+      const bool in0 = b[u] >= 0 && b[u] == base, in1 = b[u] >= 0 && b[u] == base + 1;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double t0 = v[u][c], t1 = v[u][c];
+        if (kSecond) {
+          t0 = v[u][c] - d0[c];
+          t1 = v[u][c] - d1[c];
+          t0 = t0 * t0;
+          t1 = t1 * t1;
+        }
+        s0[c] += in0 ? t0 : 0.0;
+        s1[c] += in1 ? t1 : 0.0;
+      }
+      c0 += in0 ? 1u : 0u;
+      c1 += in1 ? 1u : 0u;
+      if (b[u] >= 0 && !in0 && !in1) {
+        for (int c = 0; c < 3; ++c) {
+          const double d = kSecond ? v[u][c] - dr[c * k.nbins + b[u]] : 0.0;
+          atomicAdd(&acc[c * k.nbins + b[u]], kSecond ? d * d : v[u][c]);
+        }
+        if (!kSecond) atomicAdd(&cnt[b[u]], 1u);
+      }
     }
   }
+  rebase(-2);
   __syncthreads();
   for (int b = threadIdx.x; b < 3 * k.nbins; b += blockDim.x)
     if (acc[b] != 0.0) atomicAdd(&k.sum[b], acc[b]);
@@ -257,14 +376,23 @@ PartK part_k(const Species &s) {
   p.vz = s.vz;
   p.loc = s.loc;
   p.n = s.n_slots;
-  p.f32 = s.f32 ? 1 : 0;
   p.ney = g.m.ney;
   p.xmin = g.m.xmin;
   p.hx = g.m.hx;
   return p;
 }
 
-unsigned grid_for(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks_for(n, 256), 148 * 4)); }
+// CTAs of one wave (all resident at once), fewer for few particles
+template <class K>
+int grid_for(K kernel, size_t smem, int64_t n, unsigned *grid) {
+  int dev = 0, nsm = 0, per_sm = 0;
+  PIC_CUDA(cudaGetDevice(&dev));
+  PIC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem));
+  *grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks_for(n, 256), (int64_t)nsm * std::max(per_sm, 1)));
+  return PIC_OK;
+}
 
 // device scratch for the diagnostics, grown on demand and freed at finalize
 struct DiagScratch {
@@ -333,7 +461,7 @@ int pic_average_x(double *out) {
   const size_t bytes = (size_t)c * g.m.nnx * sizeof(double);
   if ((rc = scratch(bytes, &d))) return rc;
   k.out = static_cast<double *>(d);
-  k_average_x<<<dim3((g.m.nnx + 127) / 128, c), 128, 0, g.st>>>(k);
+  k_average_x<<<dim3((g.m.nnx + kAvgCols - 1) / kAvgCols, c), kAvgThreads, 0, g.st>>>(k);
   PIC_LAUNCHED();
   PIC_CUDA(cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, g.st));
   PIC_CUDA(cudaStreamSynchronize(g.st));
@@ -359,10 +487,13 @@ int pic_energy_spectrum(int32_t species, int32_t nbins, double e_max_ev, double 
   unsigned long long *cnt = static_cast<unsigned long long *>(d);
   PIC_CUDA(cudaMemsetAsync(cnt, 0, bytes, g.st));
   if (s.n_slots > 0) {
-    SpecK k{part_k(s), nbins, s.mass, g.v_ref, e_max_ev, v_max, nbins / e_max_ev, nbins / v_max, cnt, cnt + nbins};
+    SpecK k{part_k(s), nbins, s.mass, g.v_ref, e_max_ev, v_max, nbins / e_max_ev, nbins / v_max,
+            e_max_ev > 1e-200 ? nbins / (e_max_ev * PIC_JTOEV) : std::nan(""), cnt, cnt + nbins};
     const size_t shb = 2 * (nbins + 1) * sizeof(double) + 2 * nbins * sizeof(unsigned int);
-    PIC_CUDA(cudaFuncSetAttribute(k_spectrum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shb));
-    k_spectrum<<<grid_for(s.n_slots), 256, shb, g.st>>>(k);
+    const auto fn = s.f32 ? k_spectrum<true> : k_spectrum<false>;
+    unsigned grid = 0;
+    if ((rc = grid_for(fn, shb, s.n_slots, &grid))) return rc;
+    fn<<<grid, 256, shb, g.st>>>(k);
     PIC_LAUNCHED();
   }
   std::vector<unsigned long long> h(2 * (size_t)nbins);
@@ -394,19 +525,21 @@ int pic_velocity_moments(int32_t species, int32_t nbins, int64_t *count, double 
   double *sum = reinterpret_cast<double *>(cnt + nb), *dr = sum + 3 * nb, *th = dr + 3 * nb;
   PIC_CUDA(cudaMemsetAsync(d, 0, nb * 8 * 4, g.st));
   const size_t sh1 = 3 * nb * sizeof(double) + nb * sizeof(unsigned int), sh2 = 6 * nb * sizeof(double);
-  PIC_CUDA(cudaFuncSetAttribute(k_vmoments<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh1));
-  PIC_CUDA(cudaFuncSetAttribute(k_vmoments<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh2));
+  const auto fn1 = s.f32 ? k_vmoments<false, true> : k_vmoments<false, false>;
+  const auto fn2 = s.f32 ? k_vmoments<true, true> : k_vmoments<true, false>;
+  unsigned grid1 = 0, grid2 = 0;
+  if ((rc = grid_for(fn1, sh1, s.n_slots, &grid1)) || (rc = grid_for(fn2, sh2, s.n_slots, &grid2))) return rc;
   MomK k{part_k(s), nbins, cnt, sum, dr};
-  const unsigned grid = grid_for(s.n_slots), gdiv = (unsigned)((3 * nb + 255) / 256);
+  const unsigned gdiv = (unsigned)((3 * nb + 255) / 256);
   if (s.n_slots > 0) {
-    k_vmoments<false><<<grid, 256, sh1, g.st>>>(k);
+    fn1<<<grid1, 256, sh1, g.st>>>(k);
     PIC_LAUNCHED();
   }
   k_vmoments_div<<<gdiv, 256, 0, g.st>>>(cnt, sum, dr, nbins, 0);
   PIC_LAUNCHED();
   PIC_CUDA(cudaMemsetAsync(sum, 0, 3 * nb * sizeof(double), g.st));
   if (s.n_slots > 0) {
-    k_vmoments<true><<<grid, 256, sh2, g.st>>>(k);
+    fn2<<<grid2, 256, sh2, g.st>>>(k);
     PIC_LAUNCHED();
   }
   k_vmoments_div<<<gdiv, 256, 0, g.st>>>(cnt, sum, th, nbins, 1);

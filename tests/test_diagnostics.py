@@ -162,3 +162,44 @@ def test_output_files(tmp_path):
         assert tab.shape == (2, 4) and tab[1, 1] == tab[1, 2] + tab[1, 3]
     finally:
         sim.close()
+
+
+# runs of 64 particles a warp, the two columns a warp keeps in registers, and
+# particles in any order; counts exact, sums as above
+@pytest.mark.parametrize("prec", PRECISIONS)
+@pytest.mark.parametrize("order", ["sorted", "unsorted"])
+@pytest.mark.parametrize("n", [1, 31, 65, 2049, 40001])
+def test_binned_diagnostics_match_oracle_at_run_edges(n, order, prec):
+    cfg = deck.config("tiny", ncx=48, ncy=20, Lx=0.03, Ly=0.0125, objects=[], precision=prec)
+    sim = Simulation(cfg, load=False, capacity=[n, 16], mcc=False)
+    try:
+        rng = np.random.default_rng(n)
+        m = sim.mesh
+        x, y = rng.random(n) * m.hx * 48, rng.random(n) * m.hy * 20
+        v = rng.standard_normal((3, n)) * np.array([[1.0], [0.05], [1.0]])
+        v[:, ::7] = 0.25  # values on the edges of the bins below
+        sim.upload(0, x, y, *[np.ascontiguousarray(c) for c in v])
+        if order == "sorted":
+            sim.sort(0)
+        parts = _live(sim, 0)
+        for nbins in (1, 2, 90, 2048):
+            cnt, drift, thermal = sim.velocity_moments(0, nbins)
+            oc, od, ot = ob.velocity_moments(parts, nbins)
+            assert np.array_equal(cnt, oc)
+            for g, o in ((drift, od), (thermal, ot)):
+                assert np.all(np.abs(g - o) <= 1e-12 * max(np.abs(o).max(), np.abs(v).max()))
+        mass, vref = sim.species[0][1], sim.scales["v_ref"]
+        e = 0.5 * mass * (parts["vx"][0] ** 2 + parts["vy"][0] ** 2 + parts["vz"][0] ** 2) * vref * vref / 1.6022e-19
+        for nbins, e_max, v_max in ((1, 4.0, 1.0), (64, 2.0 * float(e), 4.0), (4096, 20.0, 8.0), (100, 1e-3, 1e-3)):
+            ce, cv = sim.energy_spectrum(0, nbins, e_max, v_max)
+            oe, ov = ob.energy_spectrum(parts, mass, vref, nbins, e_max, v_max)
+            assert np.array_equal(ce, oe) and np.array_equal(cv, ov), nbins
+        sim.get_par_chg()
+        prof = sim.average_x()
+        rho = sim.field("rho_e").reshape(m.nnx, m.nny)
+        s = np.zeros(m.nnx)
+        for j in range(m.nny):  # node order
+            s = s + rho[:, j]
+        assert np.array_equal(prof["Rho_ele"], (s / m.nny) * cfg.n0)
+    finally:
+        sim.close()
