@@ -22,6 +22,7 @@
 #include <string>
 
 #include "../../include/picgpu.h"
+#include "div_dev.h"
 #include "pic_common.h"
 
 namespace pic {
@@ -45,35 +46,122 @@ __global__ void k_na_clear(unsigned long long *acc, int64_t nn) {
   if (i < nn) acc[i] = 0ull;
 }
 
-__global__ void k_na_deposit(int nnx, int nny, double xmin, double ymin, double hx, double hy, int64_t n,
-                             const double *__restrict__ x, const double *__restrict__ y,
-                             const int32_t *__restrict__ loc, unsigned long long *acc) {
-  int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  if (loc && loc[p] < 0) return;  // absorbed slot
-  const int nex = nnx - 1, ney = nny - 1;
-  double px = x[p], py = y[p];
-  double rxp = (px - xmin) / hx, ryp = (py - ymin) / hy;
-  int i = (int)rxp + 1, j = (int)ryp + 1;
-  if (i == nnx) i = nnx - 1;
-  if (j == nny) j = nny - 1;
-  if (!(rxp >= 0.0) || !(ryp >= 0.0) || i < 1 || j < 1 || i > nex || j > ney) return;
-  int ie = i - 1, je = j - 1;
-  double x1 = xmin + hx * ie, x2 = xmin + hx * (ie + 1);
-  double y1 = ymin + hy * je, y2 = ymin + hy * (je + 1);
-  double dx = (px - x1) / (x2 - x1);
-  double dy = (py - y1) / (y2 - y1);
-  double xc = 1.0 - dx, yc = 1.0 - dy;
-  double W[4] = {xc * yc, dx * yc, dx * dy, xc * dy};
-  int64_t n1 = (int64_t)ie * nny + je;
-  int64_t nodes[4] = {n1, n1 + nny, n1 + nny + 1, n1 + 1};
-  // corner 2 takes the rest of the particle's 2^40, as pic_get_par_chg does
-  long long q[4];
-  q[0] = __double2ll_rn(W[0] * PIC_Q_SCALE);
-  q[1] = __double2ll_rn(W[1] * PIC_Q_SCALE);
-  q[3] = __double2ll_rn(W[3] * PIC_Q_SCALE);
-  q[2] = (1ll << 40) - ((q[0] + q[1]) + q[3]);
-  for (int c = 0; c < 4; ++c) atomicAdd(acc + nodes[c], (unsigned long long)q[c]);
+// Sums over lanes [lane, seg_end] of one segment, toward its head.
+__device__ __forceinline__ void seg_sums4(long long (&v)[4], int lane, int seg_end, int maxlen) {
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    if (off >= maxlen) break;
+    const bool take = lane + off <= seg_end;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const long long o = __shfl_down_sync(0xffffffffu, v[c], off);
+      if (take) v[c] += o;
+    }
+  }
+}
+
+__device__ __forceinline__ void na_add(unsigned long long *acc, int n1, int nny, const long long (&q)[4]) {
+  atomicAdd(acc + n1, (unsigned long long)q[0]);
+  atomicAdd(acc + n1 + nny, (unsigned long long)q[1]);
+  atomicAdd(acc + n1 + nny + 1, (unsigned long long)q[2]);
+  atomicAdd(acc + n1 + 1, (unsigned long long)q[3]);
+}
+
+// Four consecutive particles a thread.  Bound by the atomics where each
+// particle adds its own (3M cell-sorted particles on 257 x 200 nodes: 12M adds
+// on 51,400 addresses, 158 us); callers mostly keep particles in cell order,
+// so a thread sums its particles in registers while they stay in one element,
+// and the warp sums the threads' last runs by segments of equal elements,
+// unless nearly every lane holds another one (unsorted particles: then each
+// adds its own, as many atomics as before).  The four quotients a particle
+// needs are products (div_dev.h, the same bits as the divisions).
+// A call with those particles: 158 -> 38 us.
+constexpr int kNaRun = 4;
+
+__global__ void __launch_bounds__(256) k_na_deposit(int nnx, int nny, double xmin, double ymin, double hx, double hy,
+                                                    int64_t n, const double *__restrict__ x,
+                                                    const double *__restrict__ y, const int32_t *__restrict__ loc,
+                                                    int vec, unsigned long long *acc) {
+  const int64_t p0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kNaRun;
+  const int nex = nnx - 1, ney = nny - 1, lane = threadIdx.x & 31;
+  const double rhx = pic::recip_const(hx), rhy = pic::recip_const(hy);
+  double px[kNaRun], py[kNaRun];
+  int lc[kNaRun];
+  if (vec && p0 + kNaRun <= n) {  // 16-byte aligned arrays
+#pragma unroll
+    for (int k = 0; k < kNaRun; k += 2) {
+      const double2 a = *reinterpret_cast<const double2 *>(x + p0 + k), b = *reinterpret_cast<const double2 *>(y + p0 + k);
+      px[k] = a.x;
+      px[k + 1] = a.y;
+      py[k] = b.x;
+      py[k + 1] = b.y;
+    }
+    const int4 l = loc ? *reinterpret_cast<const int4 *>(loc + p0) : make_int4(0, 0, 0, 0);
+    lc[0] = l.x;
+    lc[1] = l.y;
+    lc[2] = l.z;
+    lc[3] = l.w;
+  } else {
+#pragma unroll
+    for (int k = 0; k < kNaRun; ++k) {
+      const bool in = p0 + k < n;
+      px[k] = in ? x[p0 + k] : 0.0;
+      py[k] = in ? y[p0 + k] : 0.0;
+      lc[k] = !in ? -1 : loc ? loc[p0 + k] : 0;
+    }
+  }
+  int key = -1;  // the run's first node
+  long long q[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < kNaRun; ++k) {
+    if (lc[k] < 0) continue;  // absorbed slot
+    bool exact = true;
+    double rxp = pic::div_const(px[k] - xmin, hx, rhx, exact), ryp = pic::div_const(py[k] - ymin, hy, rhy, exact);
+    if (!exact) {
+      rxp = (px[k] - xmin) / hx;
+      ryp = (py[k] - ymin) / hy;
+    }
+    int i = (int)rxp + 1, j = (int)ryp + 1;
+    if (i == nnx) i = nnx - 1;
+    if (j == nny) j = nny - 1;
+    if (!(rxp >= 0.0) || !(ryp >= 0.0) || i < 1 || j < 1 || i > nex || j > ney) continue;
+    const int ie = i - 1, je = j - 1;
+    const double x1 = xmin + hx * ie, x2 = xmin + hx * (ie + 1);
+    const double y1 = ymin + hy * je, y2 = ymin + hy * (je + 1);
+    exact = true;
+    double dx = pic::div_const(px[k] - x1, x2 - x1, pic::recip_near(x2 - x1, rhx), exact);
+    double dy = pic::div_const(py[k] - y1, y2 - y1, pic::recip_near(y2 - y1, rhy), exact);
+    if (!exact || fabs((x2 - x1) - hx) > 1e-9 * hx || fabs((y2 - y1) - hy) > 1e-9 * hy) {
+      dx = (px[k] - x1) / (x2 - x1);
+      dy = (py[k] - y1) / (y2 - y1);
+    }
+    const double xc = 1.0 - dx, yc = 1.0 - dy;
+    const int n1 = ie * nny + je;
+    if (n1 != key) {
+      if (key >= 0) na_add(acc, key, nny, q);
+      key = n1;
+      q[0] = q[1] = q[2] = q[3] = 0;
+    }
+    // corner 2 takes the rest of the particle's 2^40, as pic_get_par_chg does
+    const long long q0 = __double2ll_rn((xc * yc) * PIC_Q_SCALE), q1 = __double2ll_rn((dx * yc) * PIC_Q_SCALE);
+    const long long q3 = __double2ll_rn((xc * dy) * PIC_Q_SCALE);
+    q[0] += q0;
+    q[1] += q1;
+    q[3] += q3;
+    q[2] += (1ll << 40) - ((q0 + q1) + q3);
+  }
+  const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+  const bool head = lane == 0 || key != prev;
+  const unsigned heads = __ballot_sync(0xffffffffu, head);
+  if (__popc(heads) <= 20) {
+    const unsigned above = lane == 31 ? 0u : (heads & ~((2u << lane) - 1u));
+    const int seg_end = above ? __ffs(above) - 2 : 31;
+    const int maxlen = (int)__reduce_max_sync(0xffffffffu, head ? (unsigned)(seg_end - lane + 1) : 0u);
+    seg_sums4(q, lane, seg_end, maxlen);
+    if (head && key >= 0) na_add(acc, key, nny, q);
+  } else if (key >= 0) {
+    na_add(acc, key, nny, q);
+  }
 }
 
 __global__ void k_na_normalize(const unsigned long long *acc, const double *__restrict__ vol, double wq,
@@ -130,7 +218,9 @@ extern "C" int pic_deposit_noalloc(int32_t nnx, int32_t nny, double xmin, double
   const double hx = (xmax - xmin) / (nnx - 1), hy = (ymax - ymin) / (nny - 1);
   k_na_clear<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, nn);
   if (n > 0)
-    k_na_deposit<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nnx, nny, xmin, ymin, hx, hy, n, x, y, loc, acc);
+    k_na_deposit<<<(unsigned)((n + 256 * kNaRun - 1) / (256 * kNaRun)), 256, 0, st>>>(
+        nnx, nny, xmin, ymin, hx, hy, n, x, y, loc,
+        (((uintptr_t)x | (uintptr_t)y | (uintptr_t)loc) & 15) == 0, acc);
   k_na_normalize<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, cell_volume, weight_charge, L_ref, n_ref,
                                                                 rho_out, nn);
   e = cudaGetLastError();

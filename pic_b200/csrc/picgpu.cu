@@ -29,6 +29,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "div_dev.h"
 #include "pic_ctx.h"
 
 namespace pic {
@@ -1779,28 +1780,6 @@ __device__ __forceinline__ bool poll_tagged(const bool (&want)[N], const ulonglo
     }
     if (__any_sync(0xffffffffu, stop)) return false;
   }
-}
-
-// a / d with y = 1/d rounded to nearest (NaN where d is out of the range in
-// which this holds), the same bits as the division: a correction of a y makes
-// it the quotient to within its last place, and by Markstein's theorem (IBM
-// J. Res. Dev. 34, 1990) one more with the exact remainder rounds correctly.
-// Five dependent operations and no branch for the Jacobi preconditioner's
-// divisions by constants; zeros (every Dirichlet node) keep their sign.
-// exact is cleared where the caller has to divide.
-__device__ __forceinline__ double div_const(double a, double d, double y, bool &exact) {
-  double q = a * y;
-  const double zero = q;
-  q = fma(fma(-q, d, a), y, q);
-  q = fma(fma(-q, d, a), y, q);
-  const double m = fabs(a);
-  exact = exact && ((m > 1e-250 && m < 1e250 && y == y) || m == 0.0);
-  return m == 0.0 ? zero : q;
-}
-
-__device__ __forceinline__ double recip_const(double d) {
-  const double m = fabs(d);
-  return m > 1e-40 && m < 1e40 ? 1.0 / d : __longlong_as_double(0x7ff8000000000000ll);
 }
 
 // A p at one node of the window; i: the node's slot.  The coefficients and
