@@ -42,15 +42,14 @@ struct MgK {
   MgLevel lv[PIC_MG_MAX_LEVELS];
 };
 
-// (i, j) of node m, a node of the 3x3 neighbourhood of node n = (I, J) on a
-// grid of ny nodes per column, without an integer division: m - n = a ny + c
-// with a, c in {-1, 0, 1} (ny >= 3).
-__device__ __forceinline__ void mg_nb_ij(int64_t n, int I, int J, int64_t m, int ny, int &i, int &j) {
-  const int64_t d = m - n;
-  const int a = d >= ny - 1 ? 1 : (d <= 1 - ny ? -1 : 0);
-  i = I + a;
-  j = J + (int)(d - (int64_t)a * ny);
-}
+// Loads below are never behind a test: positions outside the grid read the
+// nearest node inside and carry the weight or coefficient 0 (which leaves a
+// sum as it is), and interpolation has one form for all parities.  A stencil
+// is then one round of loads in flight; with a branch a position it was nine
+// rounds, one after the other (up- and down-sweeps of the 129^2 level 5 us
+// each, of which 1.4 the barrier).
+
+__device__ __forceinline__ int mg_clamp(int v, int n) { return v < 0 ? 0 : (v >= n ? n - 1 : v); }
 
 // r_l[I,J] = sum over the 3x3 finer nodes around (2I, 2J) of w_x w_y t[f],
 // w = 1 at the centre and 1/2 beside it (P^T of bilinear interpolation);
@@ -58,52 +57,47 @@ __device__ __forceinline__ void mg_nb_ij(int64_t n, int I, int J, int64_t m, int
 template <class T>
 __device__ __forceinline__ double mg_restrict(const T *__restrict__ tf, int nxf, int nyf, int I, int J) {
   const int i0 = 2 * I, j0 = 2 * J;
+  double t[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q)
+    t[q] = (double)tf[(int64_t)mg_clamp(i0 + q / 3 - 1, nxf) * nyf + mg_clamp(j0 + q % 3 - 1, nyf)];
   double s = 0.0;
 #pragma unroll
-  for (int a = -1; a <= 1; ++a) {
-    const int i = i0 + a;
-    if (i < 0 || i >= nxf) continue;
-    const double wa = a == 0 ? 1.0 : 0.5;
-#pragma unroll
-    for (int c = -1; c <= 1; ++c) {
-      const int j = j0 + c;
-      if (j < 0 || j >= nyf) continue;
-      const double w = c == 0 ? wa : 0.5 * wa;
-      s = fma(w, (double)tf[(int64_t)i * nyf + j], s);
-    }
+  for (int q = 0; q < 9; ++q) {
+    const int a = q / 3 - 1, c = q % 3 - 1, i = i0 + a, j = j0 + c;
+    const double w = (a == 0 ? 1.0 : 0.5) * (c == 0 ? 1.0 : 0.5);
+    s = fma(i >= 0 && i < nxf && j >= 0 && j < nyf ? w : 0.0, t[q], s);
   }
   return s;
 }
 
-// (P e)[i,j] on the finer grid from the coarser level's e (nxc x nyc):
-// bilinear, the coarse nodes i/2 (even i) or (i-1)/2 and (i+1)/2 (odd i)
+// (P e)[i,j] on the finer grid from the coarser level's e (nyc nodes a
+// column): bilinear, the mean of the coarse nodes i/2 (even i, twice) or
+// (i-1)/2 and (i+1)/2 (odd i), and the same in j.  Sums of equal values and
+// factors of 1/4 are exact, so every parity gets the bits of its own formula.
 __device__ __forceinline__ double mg_prolong(const double *__restrict__ e, int nyc, int i, int j) {
   const int I = i >> 1, J = j >> 1;
-  const bool ox = i & 1, oy = j & 1;
-  const double *p = e + (int64_t)I * nyc + J;
-  if (!ox && !oy) return p[0];
-  if (ox && !oy) return 0.5 * (p[0] + p[nyc]);
-  if (!ox && oy) return 0.5 * (p[0] + p[1]);
-  return 0.25 * ((p[0] + p[nyc]) + (p[1] + p[nyc + 1]));
+  const double *p = e + (int64_t)I * nyc + J, *p1 = p + (i & 1) * (int64_t)nyc;
+  const int oy = j & 1;
+  return 0.25 * ((p[0] + p1[0]) + (p[oy] + p1[oy]));
 }
 
-// A_l applied at node n = (I,J) to the values v(m) of the 9 nodes around
-// (coefficients toward nodes outside the grid are 0 and not read)
+// A_l applied at node n = (I,J) to the values v(a, c, m) of the 9 nodes m
+// around (a, c: row and column of the stencil position; coefficients toward
+// nodes outside the grid, or inactive ones, are 0)
 template <class Fv>
 __device__ __forceinline__ double mg_apply(const MgLevel &L, int I, int J, Fv v) {
   const int64_t nl = (int64_t)L.nx * L.ny, n = (int64_t)I * L.ny + J;
+  float st[9];
+  double x[9];
+#pragma unroll
+  for (int q = 0; q < 9; ++q) st[q] = L.st[q * nl + n];
+#pragma unroll
+  for (int q = 0; q < 9; ++q)
+    x[q] = v(q / 3, q % 3, (int64_t)mg_clamp(I + q / 3 - 1, L.nx) * L.ny + mg_clamp(J + q % 3 - 1, L.ny));
   double acc = 0.0;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const int i = I + a - 1;
-    if (i < 0 || i >= L.nx) continue;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const int j = J + c - 1;
-      if (j < 0 || j >= L.ny) continue;
-      acc = fma((double)L.st[(3 * a + c) * nl + n], v((int64_t)i * L.ny + j), acc);
-    }
-  }
+  for (int q = 0; q < 9; ++q) acc = fma((double)st[q], x[q], acc);
   return acc;
 }
 
@@ -126,24 +120,45 @@ __device__ __forceinline__ void mg_restrict_node(const MgLevel &L, const T *__re
 __device__ __forceinline__ double mg_smooth_val(const MgLevel &L, int64_t n) {
   const double dn = (double)L.dinv[n];
   const int I = (int)n / L.ny, J = (int)n - I * L.ny;
-  auto z = [&](int64_t m) { return L.z[m]; };
-  const double t = L.r[n] - mg_apply(L, I, J, z);
+  const double r = L.r[n];
+  const double t = r - mg_apply(L, I, J, [&](int, int, int64_t m) { return L.z[m]; });
   return dn == 0.0 ? 0.0 : t;
 }
 
-// up-sweep: y = z + P e_c (0 on inactive nodes), e = y + w D^-1 (r - A y)
+// up-sweep: y = z + P e_c, e = y + w D^-1 (r - A y).  The 3x3 nodes interpolate
+// from 3x3 coarse ones at most (two rows and columns suffice at odd I, J),
+// loaded once.  (y is not 0 on inactive nodes, whose coefficients are.)
 __device__ __forceinline__ double mg_post_val(const MgLevel &L, const double *__restrict__ ec, int nyc, double w,
                                               int64_t n) {
-  const double dn = (double)L.dinv[n];
+  const double dn = (double)L.dinv[n], r = L.r[n];
   const int I = (int)n / L.ny, J = (int)n - I * L.ny;
-  auto y = [&](int64_t m) {
-    int i, j;
-    mg_nb_ij(n, I, J, m, L.ny, i, j);
-    const double v = L.z[m] + mg_prolong(ec, nyc, i, j);
-    return L.dinv[m] != 0.0f ? v : 0.0;
-  };
-  const double yn = y(n);
-  const double e = fma(w * dn, L.r[n] - mg_apply(L, I, J, y), yn);
+  const bool eI = (I & 1) == 0, eJ = (J & 1) == 0;
+  const int nxc = (L.nx - 1) / 2 + 1, Ib = eI ? I / 2 - 1 : I / 2, Jb = eJ ? J / 2 - 1 : J / 2;
+  double P[3][3], pe[3][3];
+#pragma unroll
+  for (int q = 0; q < 9; ++q)
+    P[q / 3][q % 3] = ec[(int64_t)mg_clamp(Ib + q / 3, nxc) * nyc + mg_clamp(Jb + q % 3, nyc)];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    // coarse rows of neighbour row a: even I (0,1) (1,1) (1,2); odd I (0,0) (0,1) (1,1)
+    double C[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const double mid = eI ? P[1][c] : P[0][c];
+      C[c] = a == 0 ? P[0][c] + mid : a == 1 ? mid + P[1][c] : P[1][c] + (eI ? P[2][c] : P[1][c]);
+    }
+    const double mid = eJ ? C[1] : C[0];
+    pe[a][0] = 0.25 * (C[0] + mid);
+    pe[a][1] = 0.25 * (mid + C[1]);
+    pe[a][2] = 0.25 * (C[1] + (eJ ? C[2] : C[1]));
+  }
+  double yn = 0.0;
+  const double Ay = mg_apply(L, I, J, [&](int a, int c, int64_t m) {
+    const double y = L.z[m] + pe[a][c];
+    if (a == 1 && c == 1) yn = y;
+    return y;
+  });
+  const double e = fma(w * dn, r - Ay, yn);
   return dn == 0.0 ? 0.0 : e;
 }
 

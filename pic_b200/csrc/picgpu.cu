@@ -1501,31 +1501,37 @@ __device__ __forceinline__ unsigned int atom_add_release_gpu(unsigned int *p, un
 
 // Grid-wide barrier on a monotonic arrival counter: thread 0 of every CTA
 // adds 1 with release semantics (after the CTA barrier, so the whole CTA's
-// writes are ordered before it) and polls with acquire loads until the count
-// reaches the end of its round.  The wait is bounded: after `limit` polls the
-// CTA records the timeout in *err and leaves; every CTA then exits the solve,
-// so a lost CTA ends the kernel with an error status instead of a hang.
-// Thread 0 reads the error word once and hands it to the CTA through shared
-// memory (one global round trip per barrier instead of one per warp).
+// writes are ordered before it) and its warp polls with acquire loads until
+// the count reaches the end of its round.  The wait is bounded: after `limit`
+// polls the CTA records the timeout in *err and leaves; the others run into
+// the same wait here or at the next barrier (and look at *err now and then),
+// so a lost CTA ends the kernel with an error status instead of a hang.  The
+// kernels' last act is to look at *err, so that no result stands which a CTA
+// that left did not finish.  (Reading *err in every round instead: 3,030 ->
+// 2,540 cycles a barrier of 148 idle CTAs, one trip through L2 less.)
 __device__ __forceinline__ bool grid_barrier(unsigned int *bar, int *err, long long limit,
                                              unsigned int extra) {
-  __shared__ int s_ok;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  bool ok = true;
+  if (threadIdx.x < 32) {
     const unsigned int n = gridDim.x + extra;
-    unsigned int t = atom_add_release_gpu(bar, 1u);
-    unsigned int target = (t / n + 1u) * n;
-    long long spins = 0;
-    while ((int)(ld_acquire_gpu(bar) - target) < 0) {
+    unsigned int t = threadIdx.x == 0 ? atom_add_release_gpu(bar, 1u) : 0u;
+    t = __shfl_sync(0xffffffffu, t, 0);
+    const unsigned int target = (t / n + 1u) * n;
+    for (long long spins = 0;;) {
+      if (__all_sync(0xffffffffu, (int)(ld_acquire_gpu(bar) - target) >= 0)) break;
       if (++spins > limit) {
-        atomicExch(err, 1);
+        if (threadIdx.x == 0) atomicExch(err, 1);
+        ok = false;
+        break;
+      }
+      if ((spins & 1023) == 0 && __any_sync(0xffffffffu, *(volatile int *)err != 0)) {
+        ok = false;
         break;
       }
     }
-    s_ok = *(volatile int *)err == 0;
   }
-  __syncthreads();
-  return s_ok != 0;
+  return !__syncthreads_or(!ok);
 }
 
 // The persistent solver runs CTAs of PIC_RED_CHUNK (1024) threads, one chunk
@@ -1678,7 +1684,7 @@ __global__ void __launch_bounds__(kWide, 1) k_pcg_persist(PcgP P) {
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     S->iter = iter;
-    S->ierr = ok ? ierr : 4;
+    S->ierr = ok && *(volatile int *)P.bar_err == 0 ? ierr : 4;
     S->normR = normR;
     S->rho = rho;
     S->done = 1;
@@ -2135,7 +2141,7 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     S->iter = iter;
-    S->ierr = ok ? ierr : 4;
+    S->ierr = ok && *(volatile int *)P.bar_err == 0 ? ierr : 4;
     S->normR = normR;
     S->rho = rho;
     S->done = 1;
@@ -2517,6 +2523,9 @@ struct FcgP {
   PcgK k;                        // operator (row kinds, FP64 and FP32 coefficients)
   V *x, *r, *r2;                 // solution, residual, second residual buffer (ping-pong)
   const V *dinv;
+  // zF shares t's buffer (t is dead once it is restricted) and Q is one
+  // buffer (its old values are read by their own node only when it is
+  // rewritten): the vectors of a 1024^2 solve then stay in L2
   V *zA, *t, *zF, *P0, *P1, *Q0, *Q1;
   double *part;                  // [4][grid] partials: F p.q, F p.r, A r.r, E zF.Q
   const __half *ainv;            // coarse inverse / ainv_scale, rows padded to ainv_ld (a multiple of 8)
@@ -2590,6 +2599,18 @@ __device__ __forceinline__ V row_apply_v(const PcgK &k, int64_t n, F v) {
 // of its 16-byte group q, read consecutive doubles of a plane (no bank
 // conflicts); each warp takes rows, accumulating in FP64.  The caller
 // separates it from the writes of rc by a grid barrier.
+// 16 bytes read once an iteration: not kept in L1, first to leave L2 (the
+// 36 MB inverse would push the solver's vectors out)
+__device__ __forceinline__ uint4 ld_stream16(const uint4 *p) {
+  uint4 v;
+  asm volatile(
+      "{.reg .b64 pol; createpolicy.fractional.L2::evict_first.b64 pol, 1.0;\n"
+      "ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], pol;}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p));
+  return v;
+}
+
 template <class V>
 __device__ __forceinline__ void coarse_gemv(const FcgP<V> &F, int nc, double *s_rc, int gwarp, int nwarps,
                                             int lane) {
@@ -2607,7 +2628,7 @@ __device__ __forceinline__ void coarse_gemv(const FcgP<V> &F, int nc, double *s_
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int q = q0 + 32 * u;
-        v[u] = q < nq ? __ldg(arow + q) : make_uint4(0u, 0u, 0u, 0u);
+        v[u] = q < nq ? ld_stream16(arow + q) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -2646,6 +2667,9 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gwarp = blockIdx.x * (kWide / 32) + warp, nwarps = gridDim.x * (kWide / 32);
   const int nc = F.ncx * F.ncy;
+  // the CTA's own chunks, contiguous: a stencil's neighbour columns are mostly
+  // the CTA's own nodes too, read from L2 once and from L1 after
+  const int c0 = (int)((int64_t)blockIdx.x * nb / G), c1 = (int)((int64_t)(blockIdx.x + 1) * nb / G);
   auto barrier = [&]() { return grid_barrier(F.bar, F.bar_err, F.spin_limit, F.bar_extra); };
   // already converged (the state came from k_fcg_resid): nothing to do
   // (every CTA reads the same state)
@@ -2667,7 +2691,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       const bool upd = have_old;
       auto rnew = [&](int64_t m) { return upd ? vfma(-a, Qp[m], r[m]) : r[m]; };
       double acc_rr = 0.0;
-      for (int c = blockIdx.x; c < nb; c += gridDim.x) {
+      for (int c = c0; c < c1; ++c) {
         const int64_t base = (int64_t)c * kWide;
         const int nvalid = (int)min((int64_t)kWide, nn - base);
         const int64_t n = base + threadIdx.x;
@@ -2712,25 +2736,30 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
     if (M.L > 1) {
       // (B') multigrid V-cycle of t: restriction and down-sweeps, the dense
       // coarsest solve, up-sweeps; a grid barrier between dependent steps
-      const int64_t gtid = (int64_t)blockIdx.x * kWide + threadIdx.x, gth = (int64_t)gridDim.x * kWide;
+      // every CTA takes an equal, contiguous share of a level's nodes, two a
+      // thread at a time: both nodes' loads ahead of the stores (small levels
+      // handed out by 1024s kept 17 of 148 CTAs busy on 129^2 nodes)
+      auto each = [&](int64_t nl, double *out, auto val) {
+        const int64_t hi = (int64_t)(blockIdx.x + 1) * nl / G;
+        for (int64_t n = (int64_t)blockIdx.x * nl / G + threadIdx.x; n < hi; n += 2 * kWide) {
+          const int64_t n2 = n + kWide;
+          const double a = val(n);
+          const double b = n2 < hi ? val(n2) : 0.0;
+          out[n] = a;
+          if (n2 < hi) out[n2] = b;
+        }
+      };
       for (int l = 1; l < M.L && ok; ++l) {
         const MgLevel &L = M.lv[l];
-        const int64_t nl = (int64_t)L.nx * L.ny;
+        const int64_t nl = (int64_t)L.nx * L.ny, hi = (int64_t)(blockIdx.x + 1) * nl / G;
         const bool smoothed = l < M.L - 1;
-        for (int64_t n = gtid; n < nl; n += gth) {
+        for (int64_t n = (int64_t)blockIdx.x * nl / G + threadIdx.x; n < hi; n += kWide) {
           if (l == 1) mg_restrict_node(L, F.t, F.nnx, k.nny, omega, smoothed, n);
           else mg_restrict_node(L, M.lv[l - 1].t, M.lv[l - 1].nx, M.lv[l - 1].ny, omega, smoothed, n);
         }
         if (!(ok = barrier())) break;
         if (smoothed) {
-          // two nodes a thread at a time: both nodes' loads ahead of the stores
-          for (int64_t n = gtid; n < nl; n += 2 * gth) {
-            const int64_t n2 = n + gth;
-            const double a = mg_smooth_val(L, n);
-            const double b = n2 < nl ? mg_smooth_val(L, n2) : 0.0;
-            L.t[n] = a;
-            if (n2 < nl) L.t[n2] = b;
-          }
+          each(nl, L.t, [&](int64_t n) { return mg_smooth_val(L, n); });
           if (!(ok = barrier())) break;
         }
       }
@@ -2741,14 +2770,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
         const MgLevel &L = M.lv[l];
         const double *ec = mg_e(M, l + 1);
         const int nyc = M.lv[l + 1].ny;
-        const int64_t nl = (int64_t)L.nx * L.ny;
-        for (int64_t n = gtid; n < nl; n += 2 * gth) {
-          const int64_t n2 = n + gth;
-          const double a = mg_post_val(L, ec, nyc, omega, n);
-          const double b = n2 < nl ? mg_post_val(L, ec, nyc, omega, n2) : 0.0;
-          L.t[n] = a;
-          if (n2 < nl) L.t[n2] = b;
-        }
+        each((int64_t)L.nx * L.ny, L.t, [&](int64_t n) { return mg_post_val(L, ec, nyc, omega, n); });
       }
       if (!ok) break;
     } else if (F.coarse) {
@@ -2773,7 +2795,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       coarse_gemv(F, nc, fcg_smem, gwarp, nwarps, lane);
       if (!(ok = barrier())) break;
       // (D) prolongation
-      for (int c = blockIdx.x; c < nb; c += gridDim.x) {
+      for (int c = c0; c < c1; ++c) {
         const int64_t n = (int64_t)c * kWide + threadIdx.x;
         if (n < nn && k.row_kind[n] >= 0) {
           const int i = (int)(n / k.nny), j = (int)(n % k.nny);
@@ -2797,10 +2819,10 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       // loads, which the compiler cannot prove independent of them)
       const double *e1 = mg_e(M, 1);
       const int ny1 = M.lv[1].ny;
-      for (int c = blockIdx.x; c < nb; c += 2 * gridDim.x) {
-        const int64_t na = (int64_t)c * kWide + threadIdx.x, nb2 = na + (int64_t)gridDim.x * kWide;
+      for (int c = c0; c < c1; c += 2) {
+        const int64_t na = (int64_t)c * kWide + threadIdx.x, nb2 = na + kWide;
         const bool ua = na < nn && k.row_kind[na] >= 0;
-        const bool ub = nb2 < nn && k.row_kind[nb2] >= 0;
+        const bool ub = c + 1 < c1 && nb2 < nn && k.row_kind[nb2] >= 0;
         double pa = 0.0, pb = 0.0, za = 0.0, zb = 0.0;
         if (ua) {
           const int i = (int)na / k.nny, j = (int)na - i * k.nny;  // the grid holds < 2^31 nodes
@@ -2820,7 +2842,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
     // (E) post-smoothing and zF.Q_old (Q_old is this iteration's Ql)
     {
       double acc_zq = 0.0;
-      for (int c = blockIdx.x; c < nb; c += gridDim.x) {
+      for (int c = c0; c < c1; ++c) {
         const int64_t n = (int64_t)c * kWide + threadIdx.x;
         if (n < nn) {
           V zf = (V)0;
@@ -2851,7 +2873,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       const bool ho = have_old;
       auto pnew = [&](int64_t m) { return ho ? vfma(bt, Pl[m], F.zF[m]) : F.zF[m]; };
       double acc[2] = {0.0, 0.0};
-      for (int c = blockIdx.x; c < nb; c += gridDim.x) {
+      for (int c = c0; c < c1; ++c) {
         const int64_t n = (int64_t)c * kWide + threadIdx.x;
         if (n < nn) {
           const V pv = pnew(n);
@@ -2886,7 +2908,7 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
     S->rr = rr;
     S->best = best;
     S->best_iter = best_iter;
-    S->ierr = ok ? ierr : 7;  // 7: a grid barrier timed out
+    S->ierr = ok && *(volatile int *)F.bar_err == 0 ? ierr : 7;  // 7: a grid barrier timed out
     S->done = 1;
   }
 }
@@ -3747,11 +3769,11 @@ static int run_fcg_persist64(pic_solve_stats *stats, int *fcg_iters, int *rc_out
   F.dinv = g.d_pc_dinv;
   F.zA = g.d_pc_za;
   F.t = g.d_pc_t;
-  F.zF = g.d_z;
+  F.zF = g.d_pc_t;
   F.P0 = g.d_fcg_P;
   F.P1 = g.d_fcg_P + nn;
   F.Q0 = g.d_fcg_Q;
-  F.Q1 = g.d_fcg_Q + nn;
+  F.Q1 = g.d_fcg_Q;
   const void *fn = fcg_fn<double>();
   const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double);  // coarse_gemv's staging
   if (!g.fcg_smem_set || g.fcg_smem_set != smem) {
@@ -3916,11 +3938,11 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
       F.x = v32 + 2 * nn;
       F.zA = v32 + 3 * nn;
       F.t = v32 + 4 * nn;
-      F.zF = v32 + 5 * nn;
+      F.zF = v32 + 4 * nn;
       F.P0 = v32 + 6 * nn;
       F.P1 = v32 + 7 * nn;
       F.Q0 = v32 + 8 * nn;
-      F.Q1 = v32 + 9 * nn;
+      F.Q1 = v32 + 8 * nn;
       F.dinv = v32 + 10 * nn;
       int outer = 0, total = 0;
       for (;;) {
@@ -3976,11 +3998,11 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
     F.dinv = g.d_pc_dinv;
     F.zA = g.d_pc_za;
     F.t = g.d_pc_t;
-    F.zF = g.d_z;
+    F.zF = g.d_pc_t;
     F.P0 = g.d_fcg_P;
     F.P1 = g.d_fcg_P + nn;
     F.Q0 = g.d_fcg_Q;
-    F.Q1 = g.d_fcg_Q + nn;
+    F.Q1 = g.d_fcg_Q;
     for (;;) {
       if ((rc = launch(F, fcg_fn<double>()))) { *rc_out = rc; return 1; }
       PIC_CUDA(cudaMemcpyAsync(&hs, g.d_fcg, sizeof hs, cudaMemcpyDeviceToHost, g.st));
