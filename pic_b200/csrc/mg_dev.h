@@ -104,13 +104,16 @@ __device__ __forceinline__ double mg_apply(const MgLevel &L, int I, int J, Fv v)
 // restriction at node n of a level that is smoothed next: r = P^T t_f and
 // z = w D^-1 r (0 on inactive nodes), so the down-sweep reads z at the
 // neighbours instead of forming it from their r and D^-1
+__device__ __forceinline__ void mg_restrict_put(const MgLevel &L, double r, double w, bool smoothed, int64_t n) {
+  L.r[n] = r;
+  if (smoothed) L.z[n] = (w * r) * (double)L.dinv[n];
+}
+
 template <class T>
 __device__ __forceinline__ void mg_restrict_node(const MgLevel &L, const T *__restrict__ tf, int nxf, int nyf,
                                                  double w, bool smoothed, int64_t n) {
   const int I = (int)n / L.ny, J = (int)n - I * L.ny;  // level grids hold < 2^31 nodes
-  const double r = mg_restrict(tf, nxf, nyf, I, J);
-  L.r[n] = r;
-  if (smoothed) L.z[n] = (w * r) * (double)L.dinv[n];
+  mg_restrict_put(L, mg_restrict(tf, nxf, nyf, I, J), w, smoothed, n);
 }
 
 // The down- and up-sweep values at node n.  Every load is issued whatever

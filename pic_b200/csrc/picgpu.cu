@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <array>
 #include <map>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -2496,11 +2497,16 @@ __global__ void __launch_bounds__(PIC_RED_THREADS) k_fcg_upd(FcgK k) {
 // phases B-D are skipped.  Loads after a grid barrier are plain (L1-cached)
 // loads: the barrier's release/acquire pair orders every CTA's writes before
 // them, and a stencil reads each value up to nine times, from L1.
-// Sum over the CTA's kWide threads of NV values, in a fixed order (warp
+// threads of a persistent FCG CTA: 128 registers each hold a phase's columns
+// and the loads of the next two; with 1024 threads of 64 the phases spilled
+// (2.17 -> 2.11 ms a 1024^2 call, 10.1 -> 9.6 ms ten 512^2 mixed steps)
+constexpr int kFcgT = 512;
+
+// Sum over the CTA's kFcgT threads of NV values, in a fixed order (warp
 // butterflies, then the warp sums in warp order); result valid in thread 0.
 template <int NV>
 __device__ __forceinline__ void cta_sum(double v[NV], double *out) {
-  __shared__ double ws[NV][kWide / 32];
+  __shared__ double ws[NV][kFcgT / 32];
 #pragma unroll
   for (int q = 0; q < NV; ++q)
     for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
@@ -2512,7 +2518,7 @@ __device__ __forceinline__ void cta_sum(double v[NV], double *out) {
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
       double t = 0.0;
-      for (int w = 0; w < kWide / 32; ++w) t += ws[q][w];
+      for (int w = 0; w < kFcgT / 32; ++w) t += ws[q][w];
       out[q] = t;
     }
   __syncthreads();
@@ -2531,10 +2537,12 @@ struct FcgP {
   const __half *ainv;            // coarse inverse / ainv_scale, rows padded to ainv_ld (a multiple of 8)
   double ainv_scale;
   int ainv_ld;
+  int ainv_stream;               // the vectors fill L2: read the inverse past it
   double *rc, *ec;
   int nnx, cs, ncx, ncy, coarse;
   MgK mg;                        // multigrid V-cycle (mg.L > 1) in place of the two-level space
   double omega;
+  const int2 *tab_rows;          // per CTA: first kind and count of its explicit rows in shared memory (or null)
   FcgState *s;
   unsigned int *bar;
   int *bar_err;
@@ -2599,6 +2607,8 @@ __device__ __forceinline__ V row_apply_v(const PcgK &k, int64_t n, F v) {
 // of its 16-byte group q, read consecutive doubles of a plane (no bank
 // conflicts); each warp takes rows, accumulating in FP64.  The caller
 // separates it from the writes of rc by a grid barrier.
+constexpr int kGemvLoads = 9;  // 4225 coarse nodes: a row in two rounds
+
 // 16 bytes read once an iteration: not kept in L1, first to leave L2 (the
 // 36 MB inverse would push the solver's vectors out)
 __device__ __forceinline__ uint4 ld_stream16(const uint4 *p) {
@@ -2621,17 +2631,17 @@ __device__ __forceinline__ void coarse_gemv(const FcgP<V> &F, int nc, double *s_
   for (int row = gwarp; row < nc; row += nwarps) {
     const uint4 *arow = reinterpret_cast<const uint4 *>(F.ainv + (size_t)row * ld);
     double acc = 0.0;
-    // four loads in flight per lane before their FMAs (the row comes from
+    // nine loads in flight per lane before their FMAs (the row comes from
     // DRAM: one load at a time would make the row a chain of latencies)
-    for (int q0 = lane; q0 < nq; q0 += 4 * 32) {
-      uint4 v[4];
+    for (int q0 = lane; q0 < nq; q0 += kGemvLoads * 32) {
+      uint4 v[kGemvLoads];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < kGemvLoads; ++u) {
         const int q = q0 + 32 * u;
-        v[u] = q < nq ? ld_stream16(arow + q) : make_uint4(0u, 0u, 0u, 0u);
+        v[u] = q >= nq ? make_uint4(0u, 0u, 0u, 0u) : F.ainv_stream ? ld_stream16(arow + q) : __ldg(arow + q);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < kGemvLoads; ++u) {
         const int q = q0 + 32 * u;
         if (q >= nq) break;
         const __half2 *h = reinterpret_cast<const __half2 *>(&v[u]);
@@ -2648,8 +2658,147 @@ __device__ __forceinline__ void coarse_gemv(const FcgP<V> &F, int nc, double *s_
   }
 }
 
+// The CTA's explicit rows in shared memory (kinds [k0, k0 + rows), each
+// stencil's nine coefficients together): from global memory they were nine
+// L2 latencies' worth of waiting for every warp that meets an interface, in
+// every column of every phase.  rows 0: they did not fit.
+constexpr int kFcgTabRows = 1100;  // 79 KB: one stencil per radius of 1024 cells
+
+struct StTab {
+  const double *c;
+  int k0, rows;
+};
+
+// A row's stencil (explicit rows as stencils) applied to the 3x3 values w
+// around its node: row_apply's coefficients and order.
+template <class V>
+__device__ __forceinline__ V stencil9(const PcgK &k, const StTab &tab, int kind, const V (&w)[3][3]) {
+  V acc = (V)0;
+  if (kind < 0) return acc;
+  if (kind < k.n_mat) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      if constexpr (sizeof(V) == sizeof(double)) acc = fma(c_stencil[kind][q], w[q / 3][q % 3], acc);
+      else acc = fmaf(c_stencil32[kind][q], w[q / 3][q % 3], acc);
+    }
+  } else if (sizeof(V) == sizeof(double) && (unsigned)(kind - tab.k0) < (unsigned)tab.rows) {
+    const double *c = tab.c + 9 * (kind - tab.k0);
+#pragma unroll
+    for (int q = 0; q < 9; ++q) acc = vfma((V)c[q], w[q / 3][q % 3], acc);
+  } else {
+    V c[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      if constexpr (sizeof(V) == sizeof(double)) c[q] = k.st_tab[q * k.st_cs + kind * k.st_rs];
+      else c[q] = k.st_tab32[q * k.st_cs + kind * k.st_rs];
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) acc = vfma(c[q], w[q / 3][q % 3], acc);
+  }
+  return acc;
+}
+
+// Walks the CTA's columns [i0, i1) of the fine grid, a thread to a row: the
+// values a stencil needs are formed once per node -- the column ahead by the
+// thread of its row, from loads issued one column earlier, its neighbours'
+// by shuffles (lanes 0 and 31 load theirs) -- and kept in registers for three
+// columns: 3 loads and 4 shuffles a node where nine positions a node took 27
+// loads (phase A), and the loads run two columns ahead of the work.
+//   load(m, i, j) -> Raw, eval(Raw) -> V: the value at node m = (i, j)
+//   pre(n) -> Pre: what body needs beside, loaded as far ahead
+//   body(n, w, raw, pre): w the 3x3 values, raw the centre's own
+// Positions outside the grid read the nearest node inside (coefficient 0).
+// Rows go in blocks of 512; a last block of at most kMarchRest rows (1025 =
+// 2 x 512 + 1 rows is the common grid) is done node by node: rest(n).
+constexpr int kMarchRest = 64;
+
+// element m of an array through a 32-bit byte offset: one register for all
+// arrays of a phase (the solver takes at most kMarchMaxNodes nodes)
+constexpr int64_t kMarchMaxNodes = (int64_t)1 << 29;
+template <class T>
+__device__ __forceinline__ T &at(T *p, unsigned m) {
+  return *reinterpret_cast<T *>(const_cast<char *>(reinterpret_cast<const char *>(p)) + (unsigned)(m * (unsigned)sizeof(T)));
+}
+
+template <class V, class Load, class Eval, class Pre, class Body, class Rest>
+__device__ __forceinline__ void march(int nnx, int nny, int i0, int i1, Load load, Eval eval, Pre pre, Body body,
+                                      Rest rest) {
+  const int lane = threadIdx.x & 31;
+  // rows of a block: a power of two where little is left over (513 = 512 + 1:
+  // two groups of columns), so that no half of the CTA idles
+  int blk = kFcgT;
+  while (blk > 64 && blk > nny) blk >>= 1;
+  if (nny < kFcgT && nny - blk > kMarchRest) blk = nny;
+  for (int jb = 0; jb < nny; jb += blk) {
+    const int rows = min(blk, nny - jb);
+    if (jb > 0 && rows <= kMarchRest) {
+      for (int q = threadIdx.x; q < rows * (i1 - i0); q += kFcgT)
+        rest((i0 + q / rows) * nny + jb + q % rows);
+      break;
+    }
+    // few rows: groups of whole warps share the columns
+    const int gs = (rows + 31) & ~31, ng = kFcgT / gs, g = (int)threadIdx.x / gs, tt = (int)threadIdx.x - g * gs;
+    if (g >= ng) continue;  // whole warps
+    const int a0 = i0 + g * (i1 - i0) / ng, a1 = i0 + (g + 1) * (i1 - i0) / ng;
+    if (a0 >= a1) continue;
+    const bool valid = tt < rows;
+    const int j = jb + min(tt, rows - 1);
+    const bool edge = lane == 0 || lane == 31;
+    const int je = lane == 0 ? max(j - 1, 0) : min(j + 1, nny - 1);
+    auto spread = [&](V v, V ve, V (&o)[3]) {
+      o[1] = v;
+      o[0] = __shfl_up_sync(0xffffffffu, v, 1);
+      o[2] = __shfl_down_sync(0xffffffffu, v, 1);
+      if (lane == 0) o[0] = ve;
+      if (lane == 31) o[2] = ve;
+    };
+    auto get = [&](int i, int row) {
+      const int ic = i < 0 ? 0 : i >= nnx ? nnx - 1 : i;
+      return load((unsigned)(ic * nny + row), ic, row);
+    };
+    using Raw = decltype(load(0u, 0, 0));
+    V w[3][3];
+    // two columns ahead of the one in work: r1, p0 (the next) and r2, p1
+    Raw rm = get(a0 - 1, j), r0 = get(a0, j), r1 = get(a0 + 1, j), r2{}, em{}, e0{}, e1{}, e2{};
+    if (edge) {
+      em = get(a0 - 1, je);
+      e0 = get(a0, je);
+      e1 = get(a0 + 1, je);
+    }
+    auto p0 = pre((unsigned)(a0 * nny + j));
+    decltype(p0) p1{};
+    if (a0 + 1 < a1) {
+      r2 = get(a0 + 2, j);
+      if (edge) e2 = get(a0 + 2, je);
+      p1 = pre((unsigned)((a0 + 1) * nny + j));
+    }
+    spread(eval(rm), eval(em), w[0]);
+    spread(eval(r0), eval(e0), w[1]);
+    for (int i = a0; i < a1; ++i) {
+      spread(eval(r1), eval(e1), w[2]);
+      const Raw rc = r0;
+      const auto pc = p0;
+      r0 = r1;
+      r1 = r2;
+      e1 = e2;
+      p0 = p1;
+      if (i + 2 < a1) {
+        r2 = get(i + 3, j);
+        if (edge) e2 = get(i + 3, je);
+        p1 = pre((unsigned)((i + 2) * nny + j));
+      }
+      if (valid) body((unsigned)(i * nny + j), w, rc, pc);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        w[0][c] = w[1][c];
+        w[1][c] = w[2][c];
+      }
+    }
+  }
+}
+
 template <class V, int EX>
-__global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
+__global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
   extern __shared__ double fcg_smem[];  // the coarse right-hand side (coarse_gemv)
   const PcgK &k = F.k;
   FcgState *S = F.s;
@@ -2665,11 +2814,21 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
   int parity = 0;
   V *rc_ = F.r, *rn_ = F.r2;  // current residual, next residual
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gwarp = blockIdx.x * (kWide / 32) + warp, nwarps = gridDim.x * (kWide / 32);
+  const int gwarp = blockIdx.x * (kFcgT / 32) + warp, nwarps = gridDim.x * (kFcgT / 32);
   const int nc = F.ncx * F.ncy;
-  // the CTA's own chunks, contiguous: a stencil's neighbour columns are mostly
-  // the CTA's own nodes too, read from L2 once and from L1 after
-  const int c0 = (int)((int64_t)blockIdx.x * nb / G), c1 = (int)((int64_t)(blockIdx.x + 1) * nb / G);
+  // the CTA's own columns (explicit rows as lists: its nodes), contiguous: a
+  // stencil's neighbour columns are mostly the CTA's own nodes too
+  const int i0 = (int)((int64_t)blockIdx.x * F.nnx / G), i1 = (int)((int64_t)(blockIdx.x + 1) * F.nnx / G);
+  const int64_t n0 = (int64_t)blockIdx.x * nn / G, n1 = (int64_t)(blockIdx.x + 1) * nn / G;
+  StTab tab{fcg_smem + F.ainv_ld, 0, 0};
+  if (EX == 1 && sizeof(V) == sizeof(double) && F.tab_rows != nullptr) {
+    const int2 kr = F.tab_rows[blockIdx.x];
+    tab.k0 = kr.x;
+    tab.rows = kr.y;
+    for (int q = threadIdx.x; q < 9 * kr.y; q += kFcgT)
+      fcg_smem[F.ainv_ld + q] = k.st_tab[(q % 9) * k.st_cs + (kr.x + q / 9) * k.st_rs];
+    __syncthreads();
+  }
   auto barrier = [&]() { return grid_barrier(F.bar, F.bar_err, F.spin_limit, F.bar_extra); };
   // already converged (the state came from k_fcg_resid): nothing to do
   // (every CTA reads the same state)
@@ -2691,26 +2850,43 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       const bool upd = have_old;
       auto rnew = [&](int64_t m) { return upd ? vfma(-a, Qp[m], r[m]) : r[m]; };
       double acc_rr = 0.0;
-      for (int c = c0; c < c1; ++c) {
-        const int64_t base = (int64_t)c * kWide;
-        const int nvalid = (int)min((int64_t)kWide, nn - base);
-        const int64_t n = base + threadIdx.x;
-        if (threadIdx.x < nvalid) {
-          const V rv = rnew(n);
-          if (upd) {
-            F.x[n] = vfma(a, Pl[n], F.x[n]);
-            rn_[n] = rv;
-            acc_rr = fma((double)rv, (double)rv, acc_rr);
-          }
-          if (k.row_kind[n] < 0) {
-            F.zA[n] = (V)0;
-            F.t[n] = (V)0;
-          } else {
-            auto z1 = [&](int64_t m) { return (om * rnew(m)) * F.dinv[m]; };
-            F.zA[n] = z1(n);
-            F.t[n] = rv - row_apply_v<V, EX>(k, n, z1);
-          }
+      auto node_a = [&](int64_t n) {
+        const V rv = rnew(n);
+        if (upd) {
+          F.x[n] = vfma(a, Pl[n], F.x[n]);
+          rn_[n] = rv;
+          acc_rr = fma((double)rv, (double)rv, acc_rr);
         }
+        if (k.row_kind[n] < 0) {
+          F.zA[n] = (V)0;
+          F.t[n] = (V)0;
+        } else {
+          auto z1 = [&](int64_t m) { return (om * rnew(m)) * F.dinv[m]; };
+          F.zA[n] = z1(n);
+          F.t[n] = rv - row_apply_v<V, EX>(k, n, z1);
+        }
+      };
+      if constexpr (EX == 1) {
+        struct Raw { V r, q, d; };
+        struct Pre { V x, p; int kind; };
+        march<V>(
+            F.nnx, k.nny, i0, i1,
+            [&](unsigned m, int, int) { return Raw{at(r, m), upd ? at(Qp, m) : (V)0, at(F.dinv, m)}; },
+            [&](const Raw &v) { return (om * (upd ? vfma(-a, v.q, v.r) : v.r)) * v.d; },
+            [&](unsigned n) { return Pre{upd ? at(F.x, n) : (V)0, upd ? at(Pl, n) : (V)0, at(k.row_kind, n)}; },
+            [&](unsigned n, const V(&w)[3][3], const Raw &v, const Pre &p) {
+              const V rv = upd ? vfma(-a, v.q, v.r) : v.r;
+              if (upd) {
+                at(F.x, n) = vfma(a, p.p, p.x);
+                at(rn_, n) = rv;
+                acc_rr = fma((double)rv, (double)rv, acc_rr);
+              }
+              at(F.zA, n) = p.kind < 0 ? (V)0 : w[1][1];
+              at(F.t, n) = p.kind < 0 ? (V)0 : rv - stencil9<V>(k, tab, p.kind, w);
+            },
+            node_a);
+      } else {
+        for (int64_t n = n0 + threadIdx.x; n < n1; n += kFcgT) node_a(n);
       }
       if (upd) {
         double v[1] = {acc_rr}, o[1];
@@ -2741,8 +2917,8 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       // handed out by 1024s kept 17 of 148 CTAs busy on 129^2 nodes)
       auto each = [&](int64_t nl, double *out, auto val) {
         const int64_t hi = (int64_t)(blockIdx.x + 1) * nl / G;
-        for (int64_t n = (int64_t)blockIdx.x * nl / G + threadIdx.x; n < hi; n += 2 * kWide) {
-          const int64_t n2 = n + kWide;
+        for (int64_t n = (int64_t)blockIdx.x * nl / G + threadIdx.x; n < hi; n += 2 * kFcgT) {
+          const int64_t n2 = n + kFcgT;
           const double a = val(n);
           const double b = n2 < hi ? val(n2) : 0.0;
           out[n] = a;
@@ -2753,9 +2929,16 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
         const MgLevel &L = M.lv[l];
         const int64_t nl = (int64_t)L.nx * L.ny, hi = (int64_t)(blockIdx.x + 1) * nl / G;
         const bool smoothed = l < M.L - 1;
-        for (int64_t n = (int64_t)blockIdx.x * nl / G + threadIdx.x; n < hi; n += kWide) {
-          if (l == 1) mg_restrict_node(L, F.t, F.nnx, k.nny, omega, smoothed, n);
-          else mg_restrict_node(L, M.lv[l - 1].t, M.lv[l - 1].nx, M.lv[l - 1].ny, omega, smoothed, n);
+        const double *tf = l > 1 ? M.lv[l - 1].t : nullptr;
+        auto down = [&](int64_t n) {
+          const int I = (int)n / L.ny, J = (int)n - I * L.ny;
+          return l == 1 ? mg_restrict(F.t, F.nnx, k.nny, I, J) : mg_restrict(tf, M.lv[l - 1].nx, M.lv[l - 1].ny, I, J);
+        };
+        for (int64_t n = (int64_t)blockIdx.x * nl / G + threadIdx.x; n < hi; n += 2 * kFcgT) {
+          const int64_t n2 = n + kFcgT;
+          const double ra = down(n), rb = n2 < hi ? down(n2) : 0.0;
+          mg_restrict_put(L, ra, omega, smoothed, n);
+          if (n2 < hi) mg_restrict_put(L, rb, omega, smoothed, n2);
         }
         if (!(ok = barrier())) break;
         if (smoothed) {
@@ -2795,9 +2978,8 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       coarse_gemv(F, nc, fcg_smem, gwarp, nwarps, lane);
       if (!(ok = barrier())) break;
       // (D) prolongation
-      for (int c = c0; c < c1; ++c) {
-        const int64_t n = (int64_t)c * kWide + threadIdx.x;
-        if (n < nn && k.row_kind[n] >= 0) {
+      for (int64_t n = n0 + threadIdx.x; n < n1; n += kFcgT) {
+        if (k.row_kind[n] >= 0) {
           const int i = (int)(n / k.nny), j = (int)(n % k.nny);
           const int I = i / F.cs, J = j / F.cs;
           const double fx = (double)(i - I * F.cs) / F.cs, fy = (double)(j - J * F.cs) / F.cs;
@@ -2811,47 +2993,59 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       }
     }
     if (!(ok = barrier())) break;
-    if (M.L > 1) {
+    const bool mgrid = M.L > 1;
+    const double *e1 = mgrid ? mg_e(M, 1) : nullptr;
+    const int ny1 = mgrid ? M.lv[1].ny : 0;
+    if (EX != 1 && mgrid) {
       // (E1) zA += P e_1 once per unknown node (Dirichlet nodes keep 0), so
       // that the post-smoothing reads it at its neighbours
-      // two chunks a thread at a time: both nodes' loads are issued before
-      // either store (the stores would otherwise hold back the next chunk's
-      // loads, which the compiler cannot prove independent of them)
-      const double *e1 = mg_e(M, 1);
-      const int ny1 = M.lv[1].ny;
-      for (int c = c0; c < c1; c += 2) {
-        const int64_t na = (int64_t)c * kWide + threadIdx.x, nb2 = na + kWide;
-        const bool ua = na < nn && k.row_kind[na] >= 0;
-        const bool ub = c + 1 < c1 && nb2 < nn && k.row_kind[nb2] >= 0;
-        double pa = 0.0, pb = 0.0, za = 0.0, zb = 0.0;
-        if (ua) {
-          const int i = (int)na / k.nny, j = (int)na - i * k.nny;  // the grid holds < 2^31 nodes
-          pa = mg_prolong(e1, ny1, i, j);
-          za = (double)F.zA[na];
+      for (int64_t n = n0 + threadIdx.x; n < n1; n += kFcgT)
+        if (k.row_kind[n] >= 0) {
+          const int i = (int)n / k.nny, j = (int)n - i * k.nny;  // the grid holds < 2^31 nodes
+          F.zA[n] = (V)((double)F.zA[n] + mg_prolong(e1, ny1, i, j));
         }
-        if (ub) {
-          const int i = (int)nb2 / k.nny, j = (int)nb2 - i * k.nny;
-          pb = mg_prolong(e1, ny1, i, j);
-          zb = (double)F.zA[nb2];
-        }
-        if (ua) F.zA[na] = (V)(za + pa);
-        if (ub) F.zA[nb2] = (V)(zb + pb);
-      }
       if (!(ok = barrier())) break;
     }
-    // (E) post-smoothing and zF.Q_old (Q_old is this iteration's Ql)
+    // (E) post-smoothing of zA + P e_1 and zF.Q_old (Q_old is this iteration's Ql)
     {
       double acc_zq = 0.0;
-      for (int c = c0; c < c1; ++c) {
-        const int64_t n = (int64_t)c * kWide + threadIdx.x;
-        if (n < nn) {
+      auto put_e = [&](unsigned n, V zf, V q) {
+        at(F.zF, n) = zf;
+        if (have_old) acc_zq = fma((double)zf, (double)q, acc_zq);
+      };
+      if constexpr (EX == 1) {
+        // the coarse correction is added as a column comes in (twice in the
+        // columns next to the CTA's own)
+        // (the four coarse values as they are, for eval to sum: more registers
+        // than there are, 2.03 -> 2.11 ms a 1024^2 solve)
+        struct Raw { V z; double pe; int kind; };
+        struct Pre { V d, r, q; };
+        auto load = [&](unsigned m, int i, int j) {
+          return Raw{at(F.zA, m), mgrid ? mg_prolong(e1, ny1, i, j) : 0.0, at(k.row_kind, m)};
+        };
+        auto eval = [&](const Raw &v) { return v.kind < 0 ? (V)0 : mgrid ? (V)((double)v.z + v.pe) : v.z; };
+        march<V>(
+            F.nnx, k.nny, i0, i1, load, eval,
+            [&](unsigned n) { return Pre{at(F.dinv, n), at(r, n), have_old ? at(Ql, n) : (V)0}; },
+            [&](unsigned n, const V(&w)[3][3], const Raw &v, const Pre &p) {
+              put_e(n, v.kind < 0 ? (V)0 : vfma(om * p.d, p.r - stencil9<V>(k, tab, v.kind, w), w[1][1]), p.q);
+            },
+            [&](int64_t n) {
+              V zf = (V)0;
+              if (k.row_kind[n] >= 0) {
+                auto za = [&](int64_t m) { return eval(load((unsigned)m, (int)m / k.nny, (int)m % k.nny)); };
+                zf = vfma(om * F.dinv[n], r[n] - row_apply_v<V, EX>(k, n, za), za(n));
+              }
+              put_e((unsigned)n, zf, have_old ? Ql[n] : (V)0);
+            });
+      } else {
+        for (int64_t n = n0 + threadIdx.x; n < n1; n += kFcgT) {
           V zf = (V)0;
           if (k.row_kind[n] >= 0) {
             auto za = [&](int64_t m) { return F.zA[m]; };
             zf = vfma(om * F.dinv[n], r[n] - row_apply_v<V, EX>(k, n, za), za(n));
           }
-          F.zF[n] = zf;
-          if (have_old) acc_zq = fma((double)zf, (double)Ql[n], acc_zq);
+          put_e((unsigned)n, zf, have_old ? Ql[n] : (V)0);
         }
       }
       double v[1] = {acc_zq}, o[1];
@@ -2873,16 +3067,27 @@ __global__ void __launch_bounds__(kWide, 1) k_fcg_persist(FcgP<V> F) {
       const bool ho = have_old;
       auto pnew = [&](int64_t m) { return ho ? vfma(bt, Pl[m], F.zF[m]) : F.zF[m]; };
       double acc[2] = {0.0, 0.0};
-      for (int c = c0; c < c1; ++c) {
-        const int64_t n = (int64_t)c * kWide + threadIdx.x;
-        if (n < nn) {
-          const V pv = pnew(n);
-          const V qv = row_apply_v<V, EX>(k, n, pnew);
-          Pn[n] = pv;
-          Qn[n] = qv;
-          acc[0] = fma((double)pv, (double)qv, acc[0]);
-          acc[1] = fma((double)pv, (double)r[n], acc[1]);
-        }
+      auto put_f = [&](unsigned n, V pv, V qv, V rv) {
+        at(Pn, n) = pv;
+        at(Qn, n) = qv;
+        acc[0] = fma((double)pv, (double)qv, acc[0]);
+        acc[1] = fma((double)pv, (double)rv, acc[1]);
+      };
+      if constexpr (EX == 1) {
+        struct Raw { V z, p; };
+        struct Pre { V r; int kind; };
+        march<V>(
+            F.nnx, k.nny, i0, i1,
+            [&](unsigned m, int, int) { return Raw{at(F.zF, m), ho ? at(Pl, m) : (V)0}; },
+            [&](const Raw &v) { return ho ? vfma(bt, v.p, v.z) : v.z; },
+            [&](unsigned n) { return Pre{at(r, n), at(k.row_kind, n)}; },
+            [&](unsigned n, const V(&w)[3][3], const Raw &, const Pre &p) {
+              put_f(n, w[1][1], stencil9<V>(k, tab, p.kind, w), p.r);
+            },
+            [&](int64_t n) { put_f((unsigned)n, pnew(n), row_apply_v<V, EX>(k, n, pnew), r[n]); });
+      } else {
+        for (int64_t n = n0 + threadIdx.x; n < n1; n += kFcgT)
+          put_f((unsigned)n, pnew(n), row_apply_v<V, EX>(k, n, pnew), r[n]);
       }
       double o[2];
       cta_sum<2>(acc, o);
@@ -3133,7 +3338,7 @@ static void free_all() {
   F(g.d_phi_dir); F(g.d_cell_volume); F(g.d_rhs_fix); F(g.d_mass_q1); F(g.d_ife_mass); F(g.d_mass_rows);
   F(g.d_rf_nodes); F(g.d_rf_base);
   F(g.d_xt_ptr); F(g.d_xt_col); F(g.d_xt_val); F(g.d_row_kind); F(g.d_ex_cnt); F(g.d_ex_col);
-  F(g.d_ex_val); F(g.d_ex_val32); F(g.d_st_tab); F(g.d_st_tab32); F(g.d_fcg32); F(g.d_diag); F(g.d_ppr_kind); F(g.d_ppr_ptr); F(g.d_ppr_nodes); F(g.d_ppr_rows);
+  F(g.d_ex_val); F(g.d_ex_val32); F(g.d_st_tab); F(g.d_st_tab32); F(g.d_fcg_rows); F(g.d_fcg32); F(g.d_diag); F(g.d_ppr_kind); F(g.d_ppr_ptr); F(g.d_ppr_nodes); F(g.d_ppr_rows);
   F(g.d_ppr_h); F(g.d_phi); F(g.d_rho); F(g.d_efx); F(g.d_efy); F(g.d_efxy); F(g.d_coef); F(g.d_coef32); F(g.d_b); F(g.d_x);
   F(g.d_r); F(g.d_w); F(g.d_p[0]); F(g.d_p[1]); F(g.d_q); F(g.d_part); F(g.d_pcg); F(g.d_bar);
   F(g.d_pcg_slot); F(g.d_pcg_strip);
@@ -3695,6 +3900,11 @@ static int fcg_graph_launch(int i) {
   return PIC_OK;
 }
 
+// The coarse inverse (36 MB) is read past L2 where the nine FP64 vectors of
+// the solve and the levels below take most of its 126 MB: 1024^2 (100 MB);
+// at 512^2 (25 MB) it stays there from iteration to iteration.
+static int fcg_stream_inverse() { return g.nn * 96 > ((int64_t)64 << 20); }
+
 // the persistent FCG for this context's explicit rows
 template <class V>
 static const void *fcg_fn() {
@@ -3775,7 +3985,9 @@ static int run_fcg_persist64(pic_solve_stats *stats, int *fcg_iters, int *rc_out
   F.Q0 = g.d_fcg_Q;
   F.Q1 = g.d_fcg_Q;
   const void *fn = fcg_fn<double>();
-  const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double);  // coarse_gemv's staging
+  const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double) + g.fcg_tab_bytes;  // coarse_gemv's staging, explicit rows
+  F.tab_rows = g.d_fcg_rows;
+  F.ainv_stream = fcg_stream_inverse();
   if (!g.fcg_smem_set || g.fcg_smem_set != smem) {
     PIC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     g.fcg_smem_set = smem;
@@ -3793,7 +4005,7 @@ static int run_fcg_persist64(pic_solve_stats *stats, int *fcg_iters, int *rc_out
   for (int judged = 0;; ++judged) {
     if (int rc_ = zero_async(g.d_bar, 4 * sizeof(unsigned int), g.st)) return rc_;
     void *args[] = {&F};
-    PIC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(g.fcg_coop_grid), dim3(kWide), args, smem, g.st));
+    PIC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(g.fcg_coop_grid), dim3(kFcgT), args, smem, g.st));
     PIC_LAUNCHED();
     // the judge: the true residual of the result (r is the next start)
     k_fcg_resid<<<g.red_blocks, PIC_RED_THREADS, 0, g.st>>>(k0, g.d_dot_ticket, g.d_fcg, 0);
@@ -3907,9 +4119,11 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
     auto launch = [&](auto &F, const void *fn) -> int {
       if (int rc_ = zero_async(g.d_bar, 4 * sizeof(unsigned int), g.st)) return rc_;
       void *args[] = {&F};
-      const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double);  // coarse_gemv's staging
+      F.tab_rows = g.d_fcg_rows;
+      F.ainv_stream = fcg_stream_inverse();
+      const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double) + g.fcg_tab_bytes;  // coarse_gemv's staging, explicit rows
       PIC_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      PIC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(g.fcg_coop_grid), dim3(kWide), args, smem, g.st));
+      PIC_CUDA(cudaLaunchCooperativeKernel(fn, dim3(g.fcg_coop_grid), dim3(kFcgT), args, smem, g.st));
       PIC_LAUNCHED();
       return PIC_OK;
     };
@@ -4506,6 +4720,7 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     if ((rc = upload(&g.d_xt_val, val.data(), val.size()))) return rc;
   }
   // split A into material stencils and explicit rows
+  std::vector<int32_t> row_kind;
   {
     const int nny = m.nny;
     auto row_entries = [&](int u, std::vector<std::pair<int64_t, double>> &out) {
@@ -4657,6 +4872,7 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
       }
     }
     if ((rc = upload(&g.d_row_kind, kind.data(), kind.size()))) return rc;
+    row_kind = kind;
     if ((rc = upload(&g.d_ex_cnt, ex_cnt.data(), ex_cnt.size()))) return rc;
     if ((rc = upload(&g.d_ex_col, ex_col.data(), ex_col.size()))) return rc;
     if ((rc = upload(&g.d_ex_val, ex_val.data(), ex_val.size()))) return rc;
@@ -4848,12 +5064,33 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     g.coop_grid = (want && coop && per_sm > 0) ? std::min(g.red_blocks, per_sm * nsm) : 0;
     int per_sm_f = 0;
     int per_sm_f32 = 0;
-    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, fcg_fn<double>(), kWide, 0));
-    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f32, fcg_fn<float>(), kWide, 0));
+    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f, fcg_fn<double>(), kFcgT, 0));
+    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f32, fcg_fn<float>(), kFcgT, 0));
     per_sm_f = std::min(per_sm_f, per_sm_f32);
     const char *envf = getenv("PIC_FCG_PERSISTENT");
     const bool want_f = !(envf && envf[0] == '0');
-    g.fcg_coop_grid = (want_f && coop && per_sm_f > 0) ? std::min(g.red_blocks, per_sm_f * nsm) : 0;
+    g.fcg_coop_grid =
+        (want_f && coop && per_sm_f > 0 && nn < kMarchMaxNodes) ? std::min(g.red_blocks, nsm) : 0;
+    // the explicit rows of each CTA's columns, for its shared-memory table
+    if (g.fcg_coop_grid > 0 && g.ex_stencil) {
+      std::vector<int2> kr(g.fcg_coop_grid);
+      int most = 0;
+      for (int b = 0; b < g.fcg_coop_grid; ++b) {
+        const int64_t a0 = (int64_t)b * m.nnx / g.fcg_coop_grid * m.nny;
+        const int64_t a1 = (int64_t)(b + 1) * m.nnx / g.fcg_coop_grid * m.nny;
+        int lo = INT_MAX, hi = -1;
+        for (int64_t n = a0; n < a1; ++n)
+          if (row_kind[n] >= g.n_mat) {
+            lo = std::min(lo, row_kind[n]);
+            hi = std::max(hi, row_kind[n]);
+          }
+        kr[b] = hi < 0 ? make_int2(0, 0) : make_int2(lo, hi - lo + 1);
+        kr[b].y = std::min(kr[b].y, kFcgTabRows);  // the others come from global memory
+        most = std::max(most, kr[b].y);
+      }
+      g.fcg_tab_bytes = (size_t)most * 9 * sizeof(double);
+      if (most > 0 && (rc = upload(&g.d_fcg_rows, kr.data(), kr.size()))) return rc;
+    }
     // on-chip variant: at most eight chunks a CTA, whose window of p fits in
     // shared memory (and x and diag beside it from three chunks on)
     g.smem_grid = 0;
