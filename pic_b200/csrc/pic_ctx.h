@@ -215,6 +215,7 @@ struct Ctx {
   int32_t *d_perm = nullptr, *d_perm2 = nullptr;
   uint32_t *d_sort_id = nullptr;
   int32_t *d_scan_blk = nullptr;
+  int32_t *d_pack_cnt = nullptr, *d_pack_start = nullptr;  // download: live slots of each block of kPackSlots
   unsigned long long *d_counters = nullptr;  // misc device counters
   // MCC
   pic_gas gas;
@@ -267,6 +268,7 @@ extern Ctx g;
 // kernels launched from other translation units
 int launch_locate(Species &s, int64_t begin, int64_t end);
 int sort_species(int sidx);
+int scan_exclusive(int32_t *in, int32_t *out, int64_t n);  // on the library stream, n <= 16.7M
 int mcc_run(uint64_t step, pic_mcc_stats *stats, bool prepared = false);
 int mcc_prepare(uint64_t step);
 int fields_fence(unsigned mask);  // the library stream waits for queued copies of fields in mask

@@ -1332,26 +1332,80 @@ __global__ void k_to_mixed(MeshK m, const double *__restrict__ x, const double *
   ovz[p] = (float)vz[p];
 }
 
-// FP32 live set -> FP64 absolute positions and velocities (staging set).
-__global__ void k_from_mixed(MeshK m, const float *__restrict__ ax, const float *__restrict__ ay,
-                             const float *__restrict__ avx, const float *__restrict__ avy,
-                             const float *__restrict__ avz, const int32_t *__restrict__ loc, double *__restrict__ x,
-                             double *__restrict__ y, double *__restrict__ vx, double *__restrict__ vy,
-                             double *__restrict__ vz, int64_t n) {
-  const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const int e = loc[p];
-  double X = 0.0, Y = 0.0;
-  if (e >= 0) {
-    const int i = elem_column(m, e), j = e - i * m.ney;
-    X = m.xmin + ((double)i + (double)ax[p]) * m.hx;
-    Y = m.ymin + ((double)j + (double)ay[p]) * m.hy;
+// Packing of the live slots in slot order for the download: live slots of
+// every block of kPackSlots, their exclusive scan, then each block writes its
+// own to the staging set, FP32 offsets as absolute FP64 positions on the way.
+// (On the host it was one memcpy an element, after copies of all slots into
+// buffers of their own: 5.0 of 16.9 ms of a ten-step run of 360,000 particles.)
+constexpr int kPackSlots = 8192;
+
+__global__ void __launch_bounds__(256) k_pack_count(const int32_t *__restrict__ loc, int64_t n, int32_t *__restrict__ cnt) {
+  __shared__ int s_cnt;
+  if (threadIdx.x == 0) s_cnt = 0;
+  __syncthreads();
+  const int64_t base = (int64_t)blockIdx.x * kPackSlots;
+  int c = 0;
+  for (int q = threadIdx.x; q < kPackSlots; q += 256) c += base + q < n && loc[base + q] >= 0;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&s_cnt, c);
+  __syncthreads();
+  if (threadIdx.x == 0) cnt[blockIdx.x] = s_cnt;
+}
+
+struct PackK {
+  const double *x, *y, *vx, *vy, *vz;  // FP32 data in the same storage for F32
+  const int32_t *loc;
+  const uint32_t *id;
+  double *ox, *oy, *ovx, *ovy, *ovz;
+  int32_t *oloc;
+  uint32_t *oid;
+};
+
+template <bool F32>
+__global__ void __launch_bounds__(256) k_pack(MeshK m, PackK k, int64_t n, const int32_t *__restrict__ start) {
+  __shared__ int s_warp[2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = (int64_t)blockIdx.x * kPackSlots;
+  int64_t out = start[blockIdx.x];
+  int buf = 0;
+  for (int q0 = 0; q0 < kPackSlots && base + q0 < n; q0 += 256, buf ^= 1) {
+    const int64_t p = base + q0 + threadIdx.x;
+    const int e = p < n ? k.loc[p] : -1;
+    const unsigned live = __ballot_sync(0xffffffffu, e >= 0);
+    if (lane == 0) s_warp[buf][warp] = __popc(live);
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < 8; ++w) {
+      before += w < warp ? s_warp[buf][w] : 0;
+      total += s_warp[buf][w];
+    }
+    if (e >= 0) {
+      const int64_t o = out + before + __popc(live & ((1u << lane) - 1u));
+      if constexpr (F32) {
+        auto f = [&](const double *a) { return reinterpret_cast<const float *>(a)[p]; };
+        const int i = elem_column(m, e), j = e - i * m.ney;
+        k.ox[o] = m.xmin + ((double)i + (double)f(k.x)) * m.hx;
+        k.oy[o] = m.ymin + ((double)j + (double)f(k.y)) * m.hy;
+        k.ovx[o] = f(k.vx);
+        k.ovy[o] = f(k.vy);
+        k.ovz[o] = f(k.vz);
+      } else {
+        k.ox[o] = k.x[p];
+        k.oy[o] = k.y[p];
+        k.ovx[o] = k.vx[p];
+        k.ovy[o] = k.vy[p];
+        k.ovz[o] = k.vz[p];
+      }
+      k.oloc[o] = e;
+      k.oid[o] = k.id[p];
+    }
+    out += total;
   }
-  x[p] = X;
-  y[p] = Y;
-  vx[p] = avx[p];
-  vy[p] = avy[p];
-  vz[p] = avz[p];
+}
+
+__global__ void k_iota(uint32_t *a, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) a[i] = (uint32_t)i;
 }
 
 // ----------------------------------------------------------------------------
@@ -3528,7 +3582,7 @@ static void free_all() {
   diag_free();
   fcg_graphs_free();
   F(g.d_cell_count); F(g.d_cell_start); F(g.d_cell_fill); F(g.d_perm); F(g.d_perm2); F(g.d_sort_id);
-  F(g.d_scan_blk); F(g.d_counters); F(g.d_hist); F(g.d_sel); F(g.d_cand); F(g.d_cand_slot);
+  F(g.d_scan_blk); F(g.d_pack_cnt); F(g.d_pack_start); F(g.d_counters); F(g.d_hist); F(g.d_sel); F(g.d_cand); F(g.d_cand_slot);
   F(g.d_mcc_misc); F(g.d_mlist_key); F(g.d_mlist_slot); F(g.d_msel); F(g.d_ion_parent); F(g.d_ion_data); F(g.d_mcc_pslot); F(g.d_mcc_vel); F(g.d_ion_order);
   if (g.h_fcg) cudaFreeHost(g.h_fcg);
   for (int s = 0; s < PIC_MAX_SPECIES; ++s) {
@@ -3728,15 +3782,6 @@ static int to_mixed(Species &s) {
   std::swap(s.vx, s.vx2);
   std::swap(s.vy, s.vy2);
   std::swap(s.vz, s.vz2);
-  return PIC_OK;
-}
-
-static int from_mixed(Species &s) {
-  if (s.n_slots == 0) return PIC_OK;
-  k_from_mixed<<<blocks_for(s.n_slots, 256), 256, 0, g.st>>>(
-      mesh_k(), (const float *)s.x, (const float *)s.y, (const float *)s.vx, (const float *)s.vy,
-      (const float *)s.vz, s.loc, s.x2, s.y2, s.vx2, s.vy2, s.vz2, s.n_slots);
-  PIC_LAUNCHED();
   return PIC_OK;
 }
 
@@ -5426,6 +5471,8 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
   if ((rc = dalloc(&g.d_perm, maxcap))) return rc;
   if ((rc = dalloc(&g.d_perm2, maxcap))) return rc;
   if ((rc = dalloc(&g.d_sort_id, maxcap))) return rc;
+  if ((rc = dalloc(&g.d_pack_cnt, (size_t)blocks_for(maxcap, kPackSlots) + 1))) return rc;
+  if ((rc = dalloc(&g.d_pack_start, (size_t)blocks_for(maxcap, kPackSlots) + 1))) return rc;
   PIC_CUDA(cudaDeviceSynchronize());
   g.inited = true;
   return PIC_OK;
@@ -5451,15 +5498,15 @@ int pic_upload_particles(int32_t species, int64_t n, const double *x, const doub
   PIC_CUDA(cudaMemcpyAsync(s.vx, vx, b, cudaMemcpyHostToDevice, g.st));
   PIC_CUDA(cudaMemcpyAsync(s.vy, vy, b, cudaMemcpyHostToDevice, g.st));
   PIC_CUDA(cudaMemcpyAsync(s.vz, vz, b, cudaMemcpyHostToDevice, g.st));
-  std::vector<uint32_t> ids;
-  if (!id) {
-    ids.resize(n);
-    for (int64_t k = 0; k < n; ++k) ids[k] = (uint32_t)k;
-    id = ids.data();
-  }
   uint32_t mx = 0;
-  for (int64_t k = 0; k < n; ++k) mx = std::max(mx, id[k]);
-  PIC_CUDA(cudaMemcpyAsync(s.id, id, (size_t)n * 4, cudaMemcpyHostToDevice, g.st));
+  if (id) {
+    for (int64_t k = 0; k < n; ++k) mx = std::max(mx, id[k]);
+    PIC_CUDA(cudaMemcpyAsync(s.id, id, (size_t)n * 4, cudaMemcpyHostToDevice, g.st));
+  } else if (n > 0) {
+    mx = (uint32_t)(n - 1);
+    k_iota<<<blocks_for(n, 256), 256, 0, g.st>>>(s.id, n);
+    PIC_LAUNCHED();
+  }
   s.n_slots = n;
   s.n_live = n;
   s.next_id = n ? mx + 1 : 0;
@@ -5521,41 +5568,42 @@ int pic_download_particles(int32_t species, int64_t capacity, double *x, double 
   int rc;
   if ((rc = check_init()) || (rc = check_species(species))) return rc;
   Species &s = g.sp[species];
-  // compact on the host side: copy all slots, keep live ones in order
-  int64_t ns = s.n_slots;
-  std::vector<int32_t> hl(ns);
-  PIC_CUDA(cudaMemcpyAsync(hl.data(), s.loc, ns * 4, cudaMemcpyDeviceToHost, g.st));
-  PIC_CUDA(cudaStreamSynchronize(g.st));
-  int64_t live = 0;
-  for (int64_t k = 0; k < ns; ++k) live += hl[k] >= 0;
+  // the live slots in order: packed on the device into the staging set
+  // (nothing to pack when every slot is live), then copied
+  const int64_t ns = s.n_slots;
+  int32_t live = 0;
+  if (ns > 0) {
+    const int nblk = blocks_for(ns, kPackSlots);
+    k_pack_count<<<nblk, 256, 0, g.st>>>(s.loc, ns, g.d_pack_cnt);
+    PIC_LAUNCHED();
+    if ((rc = zero_async(g.d_pack_cnt + nblk, sizeof(int32_t), g.st))) return rc;
+    if ((rc = scan_exclusive(g.d_pack_cnt, g.d_pack_start, nblk + 1))) return rc;
+    PIC_CUDA(cudaMemcpyAsync(&live, g.d_pack_start + nblk, sizeof live, cudaMemcpyDeviceToHost, g.st));
+    PIC_CUDA(cudaStreamSynchronize(g.st));
+  }
   if (n_out) *n_out = live;
   if (live > capacity) {
     set_error("pic_download_particles: output capacity too small");
     return PIC_ERR_CAPACITY;
   }
-  auto pull = [&](const void *src, void *dst, size_t esz) -> int {
-    if (!dst) return PIC_OK;
-    std::vector<char> tmp(ns * esz);
-    PIC_CUDA(cudaMemcpy(tmp.data(), src, ns * esz, cudaMemcpyDeviceToHost));
-    int64_t o = 0;
-    for (int64_t k = 0; k < ns; ++k)
-      if (hl[k] >= 0) std::memcpy((char *)dst + (o++) * esz, tmp.data() + k * esz, esz);
-    return PIC_OK;
-  };
-  const double *sx = s.x, *sy = s.y, *svx = s.vx, *svy = s.vy, *svz = s.vz;
-  if (s.f32) {  // absolute FP64 values into the staging set
-    if ((rc = from_mixed(s))) return rc;
-    PIC_CUDA(cudaStreamSynchronize(g.st));
-    sx = s.x2;
-    sy = s.y2;
-    svx = s.vx2;
-    svy = s.vy2;
-    svz = s.vz2;
+  if (live == 0) return PIC_OK;
+  const bool pack = s.f32 || live < ns;
+  if (pack) {
+    const PackK k{s.x, s.y, s.vx, s.vy, s.vz, s.loc, s.id, s.x2, s.y2, s.vx2, s.vy2, s.vz2, s.loc2, s.id2};
+    if (s.f32) k_pack<true><<<blocks_for(ns, kPackSlots), 256, 0, g.st>>>(mesh_k(), k, ns, g.d_pack_start);
+    else k_pack<false><<<blocks_for(ns, kPackSlots), 256, 0, g.st>>>(mesh_k(), k, ns, g.d_pack_start);
+    PIC_LAUNCHED();
   }
-  if ((rc = pull(sx, x, 8)) || (rc = pull(sy, y, 8)) || (rc = pull(svx, vx, 8)) ||
-      (rc = pull(svy, vy, 8)) || (rc = pull(svz, vz, 8)) || (rc = pull(s.loc, loc, 4)) ||
-      (rc = pull(s.id, id, 4)))
-    return rc;
+  struct {
+    const void *src;
+    void *dst;
+    size_t size;
+  } const c[7] = {{pack ? s.x2 : s.x, x, 8},    {pack ? s.y2 : s.y, y, 8},       {pack ? s.vx2 : s.vx, vx, 8},
+                  {pack ? s.vy2 : s.vy, vy, 8}, {pack ? s.vz2 : s.vz, vz, 8},    {pack ? s.loc2 : s.loc, loc, 4},
+                  {pack ? s.id2 : s.id, id, 4}};
+  for (const auto &a : c)
+    if (a.dst) PIC_CUDA(cudaMemcpyAsync(a.dst, a.src, (size_t)live * a.size, cudaMemcpyDeviceToHost, g.st));
+  PIC_CUDA(cudaStreamSynchronize(g.st));
   return PIC_OK;
 }
 

@@ -102,7 +102,7 @@ __global__ void k_scan_add(int32_t *out, int64_t n, const int32_t *blk_scanned) 
   }
 }
 
-static int scan_exclusive(int32_t *in, int32_t *out, int64_t n) {
+int scan_exclusive(int32_t *in, int32_t *out, int64_t n) {
   int nb = (int)((n + 4095) / 4096);
   if (nb > 4096) {
     set_error("scan: more than 16.7M cells");
