@@ -31,7 +31,8 @@ LIBS = {
                      "headers": ["csrc/pic_ctx.h", "csrc/pic_common.h", "csrc/pic_mcc_kin.h", "csrc/ife_elem.h", "csrc/mg_dev.h", "csrc/div_dev.h",
                                  "../include/picgpu.h"],
                      "flags": ["--fmad=false"], "cutlass": False},
-    "libpicunet.so": {"sources": ["unet_conv.cu", "unet_ops.cu"], "headers": ["../include/picunet.h"],
+    "libpicunet.so": {"sources": ["unet_conv_k32.cu", "unet_conv.cu", "unet_conv_n32.cu", "unet_ops.cu"],
+                      "headers": ["../include/picunet.h", "csrc/unet_conv_tile.h"],
                       "flags": [], "cutlass": True},
 }
 

@@ -523,3 +523,29 @@ def test_params_in_one_buffer_and_replaced_ones_take_the_same_step():
         assert v["p"].data_ptr() % 16 == 0 and v["bf"].data_ptr() % 16 == 0
     used = sum(v["p"].numel() for v in nets[0].params.values())
     assert int((nets[0].params.flat["p"] != 0).sum()) <= used
+
+
+# the tiles of the convolution are chosen by channel counts (8; at most 32
+# contracted; at most 32 written) and a first-layer warp takes 16 pixels:
+# counts on both sides of each, image rows shorter and longer than 16
+@gpu
+@pytest.mark.parametrize("n,c,k,h,w", [(1, 8, 32, 1, 5), (2, 8, 40, 9, 16), (1, 8, 8, 33, 47), (1, 16, 24, 12, 9),
+                                       (1, 32, 64, 17, 20), (1, 40, 32, 8, 31), (2, 96, 32, 13, 18), (1, 72, 40, 7, 7)])
+def test_conv_tiles_match_cpu(n, c, k, h, w):
+    from pic_b200 import unet
+    import torch.nn.functional as F
+    lib = unet.load()
+    g = torch.Generator().manual_seed(3 * c + k)
+    x = _bf(torch.randn(n, h, w, c, generator=g))
+    wt = _bf(torch.randn(k, 3, 3, c, generator=g) * 0.1)
+    b = _bf(torch.randn(k, generator=g))
+    dy = _bf(torch.randn(n, h, w, k, generator=g))
+    ref = torch.relu(F.conv2d(x.double().permute(0, 3, 1, 2), wt.double().permute(0, 3, 1, 2), b.double(), padding=1))
+    y = torch.zeros(n, h, w, k, dtype=torch.bfloat16, device="cuda")
+    _conv(lib, unet.UNET_FPROP_RELU, x.cuda(), wt.cuda(), y, b.cuda())
+    assert _rel(y.double(), ref.permute(0, 2, 3, 1)) < 5e-3
+    xg = torch.nn.grad.conv2d_input((n, c, h, w), wt.double().permute(0, 3, 1, 2), dy.double().permute(0, 3, 1, 2),
+                                    padding=1)
+    dx = torch.zeros(n, h, w, c, dtype=torch.bfloat16, device="cuda")
+    _conv(lib, unet.UNET_DGRAD, dy.cuda(), wt.cuda(), dx)
+    assert _rel(dx.double(), xg.permute(0, 2, 3, 1)) < 5e-3
