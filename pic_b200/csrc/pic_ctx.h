@@ -270,9 +270,22 @@ int launch_locate(Species &s, int64_t begin, int64_t end);
 int sort_species(int sidx);
 int scan_exclusive(int32_t *in, int32_t *out, int64_t n);  // on the library stream, n <= 16.7M
 int mcc_run(uint64_t step, pic_mcc_stats *stats, bool prepared = false);
-int mcc_prepare(uint64_t step);
 int fields_fence(unsigned mask);  // the library stream waits for queued copies of fields in mask
 int zero_async(void *p, size_t bytes, cudaStream_t st);  // zero fill by a kernel (bytes, p: multiples of 4)
+// several zero fills in one launch (a step clears up to a dozen small ranges;
+// p: multiples of 16, bytes: of 4)
+struct ZeroList {
+  static constexpr int kMax = 24;
+  void *p[kMax];
+  int64_t words[kMax];
+  int n = 0;
+  void add(void *q, size_t bytes) {
+    p[n] = q;
+    words[n++] = (int64_t)(bytes / 4);
+  }
+};
+int zero_list(const ZeroList &z, cudaStream_t st);
+int mcc_prepare(uint64_t step, ZeroList *clear);  // what has to be cleared before the push is added to *clear
 int launch_spmv(const double *v, double *out);  // out = A v (solver operator)
 int coarse_setup(const pic_mesh_desc *mesh, int coarse_cells);
 int precond_apply(int full, const double *r, double *z);

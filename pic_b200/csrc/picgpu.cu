@@ -3630,6 +3630,30 @@ __global__ void k_zero(uint32_t *head, int nhead, uint4 *mid, int64_t nmid, uint
   for (int64_t i = t; i < nmid; i += stride) mid[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
+__global__ void k_zero_list(ZeroList z) {
+  uint32_t *p = static_cast<uint32_t *>(z.p[blockIdx.y]);
+  const int64_t n = z.words[blockIdx.y], n4 = n / 4;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = t; i < n4; i += stride) reinterpret_cast<uint4 *>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+  if (t < n - 4 * n4) p[4 * n4 + t] = 0u;
+}
+
+int zero_list(const ZeroList &z, cudaStream_t st) {
+  if (z.n == 0) return PIC_OK;
+  int64_t most = 0;
+  for (int k = 0; k < z.n; ++k) {
+    if ((uintptr_t)z.p[k] & 15u) {
+      set_error("zero_list: pointer must be a multiple of 16 bytes");
+      return PIC_ERR_ARG;
+    }
+    most = std::max(most, z.words[k]);
+  }
+  const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((most / 4 + 255) / 256, 148 * 8));
+  k_zero_list<<<dim3((unsigned)blocks, (unsigned)z.n), 256, 0, st>>>(z);
+  PIC_LAUNCHED();
+  return PIC_OK;
+}
+
 int zero_async(void *p, size_t bytes, cudaStream_t st) {
   if (bytes == 0) return PIC_OK;
   const uintptr_t a = (uintptr_t)p, e = a + bytes;
@@ -5794,17 +5818,21 @@ int pic_step(uint64_t step, pic_step_stats *stats) {
   // output cadence: it is deposited on steps that are multiples of
   // diag_interval (every step when diag_interval <= 1).
   const bool diag = g.P.diag_interval <= 1 || (step % (uint64_t)g.P.diag_interval) == 0;
-  if ((rc = zero_deposit(diag))) return rc;
-  if ((rc = zero_counter(1))) return rc;
+  // everything the push adds to, cleared in one launch (it was nine)
+  ZeroList clear;
   int64_t before[PIC_MAX_SPECIES];
   int64_t pushed = 0;
   for (int s = 0; s < g.ns; ++s) {
     before[s] = g.sp[s].n_live;
     pushed += before[s];
-    if ((rc = zero_counter(8 + s))) return rc;
+    clear.add(g.sp[s].q_acc, g.nn * sizeof(unsigned long long));
+    if (diag) clear.add(g.sp[s].e_acc, g.nn * sizeof(unsigned long long));
   }
+  clear.add(g.d_counters, 2 * sizeof(unsigned long long));                              // 1: outside the mesh (0 unused)
+  clear.add(g.d_counters + 8, PIC_MAX_SPECIES * sizeof(unsigned long long));            // lost, per species
   // the MCC selection of this step is built by the push itself
-  if (g.mcc_ready && g.mcc_push_select && (rc = mcc_prepare(step))) return rc;
+  if (g.mcc_ready && g.mcc_push_select && (rc = mcc_prepare(step, &clear))) return rc;
+  if ((rc = zero_list(clear, g.st))) return rc;
   PIC_CUDA(cudaEventRecord(e[6], g.st));
   g.sel_push = g.sel_step == step;
   for (int s = 0; s < g.ns; ++s)
@@ -5836,10 +5864,7 @@ int pic_step(uint64_t step, pic_step_stats *stats) {
   {  // the particles each species lost in the push, one read for all
     unsigned long long lost[PIC_MAX_SPECIES];
     if ((rc = read_counters(8, g.ns, lost))) return rc;
-    for (int s = 0; s < g.ns; ++s) {
-      g.sp[s].n_live -= (int64_t)lost[s];
-      if ((rc = zero_counter(8 + s))) return rc;
-    }
+    for (int s = 0; s < g.ns; ++s) g.sp[s].n_live -= (int64_t)lost[s];  // cleared before the next push
   }
   // 4. MCC
   pic_mcc_stats ms;
