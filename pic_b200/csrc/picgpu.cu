@@ -2711,27 +2711,31 @@ __global__ void __launch_bounds__(PIC_RED_THREADS) k_fcg_upd(FcgK k) {
 }
 
 // ---- persistent flexible CG (window 1, classical stages) -------------------
-// The whole solve in one cooperative kernel of kWide-thread CTAs: per
-// iteration six phases, separated by the bounded grid barrier of the
+// The whole solve in one cooperative kernel of kFcgT-thread CTAs: per
+// iteration the phases below, separated by the bounded grid barrier of the
 // persistent Jacobi-PCG.  Scalars (beta, alpha, r.r) are formed by every CTA
-// from the chunk partials in the canonical order, so all CTAs take the same
+// from the CTAs' partials in the same order, so all CTAs take the same
 // decisions.  Phases:
-//   (A) x += alpha P, r' = r - alpha Q (previous direction; r ping-pongs,
-//       r' is formed at the neighbours), r'.r', then pre-smoothing
-//       zA = w D^-1 r', t = r' - A zA
+//   (A) x += alpha P, r' = r - alpha Q (previous direction; r ping-pongs),
+//       r'.r', then pre-smoothing zA = w D^-1 r', t = r' - A zA
 //   (B) rc = P^T t                             (restriction, warp per coarse node)
 //   (C) ec = Ac^-1 rc                          (GEMV, warp per row)
-//   (D) zA += P ec                             (prolongation)
-//   (E) zF = zA + w D^-1 (r - A zA), zF.Q_old  (post-smoothing)
-//   (F) P_new = zF + beta P_old formed at the neighbours, Q_new = A P_new,
-//       p.q, p.r
-// Dot products are summed per thread over the CTA's chunks and once per CTA
-// (cta_sum), so warps run through their chunks without CTA-wide waits; the
-// order is fixed for a given grid, so the solve is deterministic.
-// The convergence test on r'.r' follows phase A.  Without a coarse space
-// phases B-D are skipped.  Loads after a grid barrier are plain (L1-cached)
-// loads: the barrier's release/acquire pair orders every CTA's writes before
-// them, and a stencil reads each value up to nine times, from L1.
+//   (D) zA += P ec                             (prolongation, two-level space)
+//   (E) zF = zA + w D^-1 (r - A zA), zF.Q_old  (post-smoothing; with the
+//       V-cycle zA + P e_1 is formed here, once a node, on the way in)
+//   (F) P_new = zF + beta P_old, Q_new = A P_new, p.q, p.r
+// A, E and F walk columns (march) where the operator's rows are stencils, so
+// the values a stencil reads are formed once a node.  With the V-cycle, B-D
+// are the levels' sweeps of mg_dev.h around the coarsest level's C.
+// What bounds it (1024^2, FP64): latency.  157k cycles an iteration: A and E
+// 28k each, F 18k, C 23k, the grid barriers with the CTAs' skew 60k; about
+// 200 MB cross HBM (30 us of 80).  A 14-iteration solve call 2.96 -> 2.03 ms.
+// Dot products are summed per thread over the CTA's nodes and once per CTA
+// (cta_sum); the order is fixed for a given grid, so the solve is
+// deterministic.  The convergence test on r'.r' follows phase A.  Without a
+// coarse space phases B-D are skipped.  Loads after a grid barrier are plain
+// (L1-cached) loads: the barrier's release/acquire pair orders every CTA's
+// writes before them.
 // threads of a persistent FCG CTA: 128 registers each hold a phase's columns
 // and the loads of the next two; with 1024 threads of 64 the phases spilled
 // (2.17 -> 2.11 ms a 1024^2 call, 10.1 -> 9.6 ms ten 512^2 mixed steps)
@@ -5406,8 +5410,9 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
                        : g.push_minb == 5   ? (const void *)k_push_mixed_tiled<4, 5>
                        : g.push_minb == 6   ? (const void *)k_push_mixed_tiled<4, 6>
                                             : (const void *)k_push_mixed_tiled<4>;
-      // PIC_PUSH_BULK=1 (default): the 4-stage, 5-CTA form with tiles
-      // bulk-copied by one thread and completing on mbarriers
+      // PIC_PUSH_BULK=1 (default; wherever the 4-stage, 5-CTA tiled form would
+      // run): tiles bulk-copied by one thread and completing on mbarriers,
+      // kMixStages tiles a CTA of kPairThreads threads, kMixCtas CTAs per SM
       const char *pb = getenv("PIC_PUSH_BULK");
       g.push_bulk = (pb ? atoi(pb) == 1 : g.push_bulk_default) && g.push_stages == 4 && (g.axi || g.push_minb == 5);
       if (g.push_bulk)
@@ -5423,7 +5428,8 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     // FP64 push: particle tiles (9 KB each, 3 stages = 27 KB per CTA) staged
     // through shared memory when PIC_PUSH64_TILED is 1; otherwise one
     // particle per thread loaded directly (same bits either way)
-    // (2: the tiles are bulk-copied by one thread and complete on mbarriers)
+    // (2: bulk-copied by one thread, completing on mbarriers: kF64Stages tiles
+    // a CTA of kPairThreads threads, two particles a thread)
     // test hooks of the bulk-staged pushes' bounded wait: polls of a tile's
     // mbarrier before giving up, and no copies issued at all (every wait then
     // runs out and the step reports the failure)
