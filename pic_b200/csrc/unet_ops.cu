@@ -269,16 +269,22 @@ __global__ void k_head(int64_t npix, const bf16 *__restrict__ y, const float *__
 // Four threads a pixel, eight channels each (a warp reads and writes 512
 // consecutive bytes); the channel sums meet by shuffles, then one shared add a
 // warp and channel.  93 -> 6 us at 65,536 pixels against a thread a pixel with
-// 33 colliding shared adds a thread.
+// 33 colliding shared adds a thread.  The bias gradient is one number, a sum
+// of terms of both signs over all pixels: a few CTAs form it besides, in FP64,
+// so that it is rounded 16 times in all (592 rounded adds into a running sum
+// were 1e-6 off where that sum cancels).
+constexpr int kHeadBiasCtas = 16;
+
 __global__ void __launch_bounds__(256) k_head_bwd(int64_t npix, const bf16 *__restrict__ y,
                                                   const float *__restrict__ w, const float *__restrict__ gz,
                                                   bf16 *__restrict__ dy, float *__restrict__ dw,
                                                   float *__restrict__ db) {
-  __shared__ float s[33];
-  if (threadIdx.x < 33) s[threadIdx.x] = 0.0f;
+  __shared__ float s[32];
+  __shared__ double sb[8];
+  if (threadIdx.x < 32) s[threadIdx.x] = 0.0f;
   __syncthreads();
   const int g = threadIdx.x & 3;
-  float a[8], ww[8], ab = 0.0f;
+  float a[8], ww[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     a[e] = 0.0f;
@@ -294,21 +300,31 @@ __global__ void __launch_bounds__(256) k_head_bwd(int64_t npix, const bf16 *__re
       a[e] = fmaf(gp, f[e], a[e]);
     }
     st8(dy + q * 8, f_to_v8(o));
-    ab += gp;
+  }
+  const int nb = min(kHeadBiasCtas, (int)gridDim.x);
+  if ((int)blockIdx.x < nb) {
+    const int64_t p1 = npix * (blockIdx.x + 1) / nb;
+    double ab = 0.0;
+#pragma unroll 8
+    for (int64_t p = npix * blockIdx.x / nb + threadIdx.x; p < p1; p += 256) ab += (double)gz[p];
+    for (int o = 16; o > 0; o >>= 1) ab += __shfl_xor_sync(0xffffffffu, ab, o);
+    if ((threadIdx.x & 31) == 0) sb[threadIdx.x >> 5] = ab;
   }
   for (int o = 16; o >= 4; o >>= 1) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) a[e] += __shfl_xor_sync(0xffffffffu, a[e], o);
-    ab += __shfl_xor_sync(0xffffffffu, ab, o);
   }
   if ((threadIdx.x & 31) < 4) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) atomicAdd(&s[8 * g + e], a[e]);
-    if (g == 0) atomicAdd(&s[32], ab);  // the four groups hold the same pixels' sum
   }
   __syncthreads();
   if (threadIdx.x < 32) atomicAdd(dw + threadIdx.x, s[threadIdx.x]);
-  if (threadIdx.x == 32) atomicAdd(db, s[32]);
+  if (threadIdx.x == 32 && (int)blockIdx.x < nb) {
+    double ab = 0.0;
+    for (int q = 0; q < 8; ++q) ab += sb[q];
+    atomicAdd(db, (float)ab);
+  }
 }
 
 __global__ void k_loss(int64_t npix, const float *__restrict__ z, const double *__restrict__ t,

@@ -549,3 +549,27 @@ def test_conv_tiles_match_cpu(n, c, k, h, w):
     dx = torch.zeros(n, h, w, c, dtype=torch.bfloat16, device="cuda")
     _conv(lib, unet.UNET_DGRAD, dy.cuda(), wt.cuda(), dx)
     assert _rel(dx.double(), xg.permute(0, 2, 3, 1)) < 5e-3
+
+
+# the head's bias gradient is one sum over all pixels that nearly cancels:
+# each of its parts is exact to FP64 and rounded once, then added with one
+# rounding, so it is within (parts + 1) half-ulps of the parts' absolute sum
+@gpu
+@pytest.mark.parametrize("npix", [1, 63, 64, 65, 4096, 65537])
+def test_head_bias_gradient_rounds_few_times(npix):
+    from pic_b200 import unet
+    lib = unet.load()
+    g = torch.Generator().manual_seed(npix)
+    gz = torch.randn(npix, generator=g)
+    gz -= gz.mean()
+    parts = min(16, -(-4 * npix // 256))
+    cuts = [npix * b // parts for b in range(parts + 1)]
+    exact = [gz[a:b].double().sum() for a, b in zip(cuts, cuts[1:])]
+    tol = (parts + 1) * 2.0 ** -24 * float(sum(abs(e) for e in exact)) + 1e-30
+    y = _bf(torch.randn(npix, 32, generator=g)).cuda()
+    w = torch.randn(32, generator=g).cuda()
+    dy = torch.zeros(npix, 32, dtype=torch.bfloat16, device="cuda")
+    dw, db, gzd = torch.zeros(32, device="cuda"), torch.zeros(1, device="cuda"), gz.cuda()
+    assert lib.unet_head_bwd(npix, 32, P(y), P(w), P(gzd), P(dy), P(dw), P(db), None) == 0
+    torch.cuda.synchronize()
+    assert abs(float(db) - float(sum(exact))) <= tol
