@@ -116,13 +116,14 @@ class ParamSet(dict):
         for name, t in values.items():
             at[name] = total
             total += -(-t.numel() // self.ALIGN) * self.ALIGN
-        new = lambda dtype: torch.zeros(total, dtype=dtype, device="cuda")  # noqa: E731
-        self.flat = {k: new(torch.bfloat16 if k == "bf" else torch.float32) for k in ("p", "bf", "g", "m", "v")}
+        host = torch.zeros(total)
+        for name, t in values.items():
+            host[at[name]:at[name] + t.numel()] = t.reshape(-1)
+        p = host.to("cuda")
+        self.flat = {"p": p, "bf": p.to(torch.bfloat16), **{k: torch.zeros_like(p) for k in ("g", "m", "v")}}
         for name, t in values.items():
             part = slice(at[name], at[name] + t.numel())
             self[name] = {k: f[part].view(t.shape) for k, f in self.flat.items()}
-            self[name]["p"].copy_(t)
-            self[name]["bf"].copy_(self[name]["p"].to(torch.bfloat16))
         self.places = self._places()
 
     def _places(self) -> list:
