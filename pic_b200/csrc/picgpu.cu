@@ -2728,8 +2728,8 @@ __global__ void __launch_bounds__(PIC_RED_THREADS) k_fcg_upd(FcgK k) {
 // the values a stencil reads are formed once a node.  With the V-cycle, B-D
 // are the levels' sweeps of mg_dev.h around the coarsest level's C.
 // What bounds it (1024^2, FP64): latency.  157k cycles an iteration: A and E
-// 28k each, F 18k, C 23k, the grid barriers with the CTAs' skew 60k; about
-// 200 MB cross HBM (30 us of 80).  A 14-iteration solve call 2.96 -> 2.03 ms.
+// 28k each, F 18k, C 23k, the grid barriers with the CTAs' skew 60k; 96 MB
+// cross HBM (15 us of 80).  A 14-iteration solve call 2.96 -> 2.03 ms.
 // Dot products are summed per thread over the CTA's nodes and once per CTA
 // (cta_sum); the order is fixed for a given grid, so the solve is
 // deterministic.  The convergence test on r'.r' follows phase A.  Without a
