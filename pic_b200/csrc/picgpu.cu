@@ -59,8 +59,8 @@ struct FieldK {
 // ci, cj: the element's column and row (0-based), set when it is found
 __device__ __forceinline__ int locate_elem(const MeshK &m, double x, double y, int &ci, int &cj) {
   // InjectPositioning.f90:13-22: i = INT((x - dxmin)/dx) + 1 (1-based).  (The
-  // push's quotients as products by known reciprocals, div_dev.h: 2.87 ->
-  // 2.97 ms for 101M particles, a longer chain where latency bounds.)
+  // push's quotients as products by known reciprocals, div_dev.h: 2.91 ->
+  // 3.05 ms for 101M particles, a longer chain where latency bounds.)
   double rxp = (x - m.xmin) / m.hx;
   double ryp = (y - m.ymin) / m.hy;
   int i = (int)rxp + 1;
@@ -512,17 +512,16 @@ __device__ __forceinline__ void weights_axi(const MeshK &m, int e, double x, dou
 
 // One live FP64 particle p (element e, position and velocity as loaded):
 // gather E (old element), leapfrog push, wall/object absorption, locate;
-// leaves the particle's new state in x, y, vx, vy and e (the element to
-// store) and returns what the warp deposit needs.
+// writes the particle back and returns what the warp deposit needs.
 // AXI (delta = 1, MoveOne.f90:213-263): x = z, y = r and the velocity held in
 // the particle's own frame (vx = v_z, vy = v_r, vz = v_theta); after the kick
 // the transverse move X = r + dt v_r, Y = dt v_theta gives r' = |(X, Y)| and
 // (v_r, v_theta) is rotated into the new frame by (X, Y)/r'; the deposit
 // weights are weights_axi.
 template <bool AXI>
-__device__ __forceinline__ void push_fp64_core(const MeshK &m, const FieldK &f, const PushK &prm, const SpK &s,
-                                               int64_t p, int &e, double &x, double &y, double &vx, double &vy,
-                                               int &key, double W[4], int nodes[4], double &energy, bool &lost) {
+__device__ __forceinline__ void push_fp64_one(const MeshK &m, const FieldK &f, const PushK &prm, const SpK &s,
+                                              int64_t p, int e, double x, double y, double vx, double vy,
+                                              int &key, double W[4], int nodes[4], double &energy, bool &lost) {
   int en = -2;          // the new element, once located
   int ci = 0, cj = 0;   // and its column and row
   if (prm.do_push) {
@@ -591,17 +590,21 @@ __device__ __forceinline__ void push_fp64_core(const MeshK &m, const FieldK &f, 
       en = locate_elem(m, x, y, ci, cj);
       if ((en < 0 || m.elem_near[en]) && absorbed_by_object(x, y)) lost = true;
     }
+    s.x[p] = x;
+    s.y[p] = y;
+    s.vx[p] = vx;
+    s.vy[p] = vy;
   }
   if (lost) {
-    e = -1;
+    s.loc[p] = -1;
   } else if (prm.do_deposit) {
     if (en == -2) en = locate_elem(m, x, y, ci, cj);
     if (en < 0) {
       atomicAdd(s.bad, 1ull);
-      e = -1;
+      s.loc[p] = -1;
       lost = true;
     } else {
-      e = en;
+      s.loc[p] = en;
       key = en;
       if (AXI) {
         weights_axi(m, en, x, y, W, nodes);
@@ -619,21 +622,6 @@ __device__ __forceinline__ void push_fp64_core(const MeshK &m, const FieldK &f, 
 
 // One particle per thread, loaded directly: push_fp64_one, then the warp's
 // fixed-point deposit of weight and weight*energy.
-// The same for the kernels that take one particle a thread: stored where it was.
-template <bool AXI>
-__device__ __forceinline__ void push_fp64_one(const MeshK &m, const FieldK &f, const PushK &prm, const SpK &s,
-                                              int64_t p, int e, double x, double y, double vx, double vy,
-                                              int &key, double W[4], int nodes[4], double &energy, bool &lost) {
-  push_fp64_core<AXI>(m, f, prm, s, p, e, x, y, vx, vy, key, W, nodes, energy, lost);
-  if (prm.do_push) {
-    s.x[p] = x;
-    s.y[p] = y;
-    s.vx[p] = vx;
-    s.vy[p] = vy;
-  }
-  if (lost || prm.do_deposit) s.loc[p] = e;
-}
-
 template <bool AXI>
 __global__ void __launch_bounds__(256, 4) k_push(MeshK m, FieldK f, PushK prm, SpK s) {
   int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -873,8 +861,8 @@ __global__ void __launch_bounds__(256, 4) k_push_mixed(MeshK m, const float *__r
 // one.  cp.async.wait_group is a hardware wait on the CTA's own copies.
 constexpr int kPushTile = 256;
 constexpr int kMixCtas = 8;
-constexpr int kF64Stages = 2, kMixStages = 3;   // tile ring of the bulk-staged pushes
-constexpr int kPairThreads = kPushTile / 2;  // the bulk-staged pushes take two particles a thread
+constexpr int kMixStages = 3;                // tile ring of the mixed bulk-staged push
+constexpr int kPairThreads = kPushTile / 2;  // which takes two particles a thread
 struct __align__(16) PushTile {
   int32_t loc[kPushTile];
   float ax[kPushTile], ay[kPushTile], vx[kPushTile], vy[kPushTile];
@@ -1043,17 +1031,17 @@ __global__ void __launch_bounds__(256, 4) k_push_tiled(MeshK m, FieldK f, PushK 
 // FP64 push with bulk-copied tiles: one thread issues five 1-D
 // cp.async.bulk copies per 256-particle tile (x, y, vx, vy: 2 KB each; the
 // elements: 1 KB), which complete on the stage's mbarrier; the other threads
-// only wait on it, so no thread computes copy addresses.  A thread takes two
-// consecutive particles, one after the other and in place in the tile (in
-// registers they spilled), stores both with 16-byte stores and hands both to
-// one pair_deposit: bound by instructions and their latency (DRAM 27%), and
-// the segmented warp sums were their largest part.  2.91 -> 2.87 ms for 101M
-// particles against one a thread; both of a pair in flight at once (94
-// registers, 5 CTAs of 128) 3.14.  Whole tiles are
+// only wait on it, so no thread computes copy addresses.  Whole tiles are
 // copied, the last one too: the particle arrays are allocated in whole
 // tiles and slots at or beyond n are never used.  The wait is bounded: a
 // tile not complete after `limit` polls sets *s.fail, and the CTA leaves at
 // the next tile boundary.  The per-particle code is k_push's, bit for bit.
+// One particle a thread, which only reads the tile.  (Two, pushed in place in
+// the tile and deposited together, as the mixed-precision push does with
+// registers to spare: the stores into the tile want a proxy fence of every
+// thread before its stage is refilled, and with it the pair gave 2.948 ->
+// 2.944 ms at 101M particles, but 2.35 -> 2.38 at 66.9M r-z ones, 0.303 ->
+// 0.318 at 8.4M, and 10 -> 14 us a launch below 10^5.)
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *b, unsigned count) {
@@ -1096,7 +1084,7 @@ __device__ __forceinline__ void push_tile64_bulk(PushTile64 *T, uint64_t *b, con
 }
 
 template <int S, bool AXI, int MINB = 4>
-__global__ void __launch_bounds__(kPairThreads, 2 * MINB) k_push_bulk(MeshK m, FieldK f, PushK prm, SpK s, int64_t ntiles,
+__global__ void __launch_bounds__(256, MINB) k_push_bulk(MeshK m, FieldK f, PushK prm, SpK s, int64_t ntiles,
                                                       long long limit, int skip_copies) {
   extern __shared__ __align__(16) unsigned char push_smem[];
   PushTile64 *T = reinterpret_cast<PushTile64 *>(push_smem);
@@ -1136,59 +1124,22 @@ __global__ void __launch_bounds__(kPairThreads, 2 * MINB) k_push_bulk(MeshK m, F
       s_fail = 1;
       atomicAdd(s.fail, 1ull);
     }
-    PushTile64 &C = T[st];
-    const int q0 = 2 * threadIdx.x;  // the thread's pair, pushed in place in the tile
-    const int64_t p = t * kPushTile + q0;
-    bool in = false;
-    int keys[2];
-    long long qs[2][4];
-    unsigned gone = 0;
-#pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t pid = push_select_id(s, p + h);  // issued early: used after the push
-      int key = -1, e = ready && p + h < s.n ? C.loc[q0 + h] : -1;
-      double W[4] = {0, 0, 0, 0};
-      int nodes[4] = {0, 0, 0, 0};
-      double energy = 0.0;
-      bool lost = false;
-      if (e >= 0) {
-        double x = C.x[q0 + h], y = C.y[q0 + h], vx = C.vx[q0 + h], vy = C.vy[q0 + h];
-        push_fp64_core<AXI>(m, f, prm, s, p + h, e, x, y, vx, vy, key, W, nodes, energy, lost);
-        C.x[q0 + h] = x;
-        C.y[q0 + h] = y;
-        C.vx[q0 + h] = vx;
-        C.vy[q0 + h] = vy;
-        C.loc[q0 + h] = e;
-        in = true;
-      }
-      if (prm.do_energy) {  // diagnostic steps: charge and energy, particle by particle
-        warp_deposit<!AXI>(s, lane, key, W, nodes, energy, lost, prm.do_deposit, prm.do_energy);
-      } else {
-        gone += __popc(__ballot_sync(0xffffffffu, lost));
-        // corners 0, 1, 3 (and 2)
-        const long long c0 = __double2ll_rn(W[0] * PIC_Q_SCALE), c1 = __double2ll_rn(W[1] * PIC_Q_SCALE);
-        const long long c3 = __double2ll_rn(W[3] * PIC_Q_SCALE), c2 = AXI ? __double2ll_rn(W[2] * PIC_Q_SCALE) : 0;
-        if (h) {
-          qs[1][0] = c0; qs[1][1] = c1; qs[1][2] = c3; qs[1][3] = c2; keys[1] = key;
-        } else {
-          qs[0][0] = c0; qs[0][1] = c1; qs[0][2] = c3; qs[0][3] = c2; keys[0] = key;
-        }
-      }
-      push_select_cta(s, key, p + h, pid, sel_buf);
+    const PushTile64 &C = T[st];
+    const int64_t p = t * kPushTile + threadIdx.x;
+    const uint32_t pid = push_select_id(s, p);  // issued early: used after the push
+    int key = -1;
+    double W[4] = {0, 0, 0, 0};
+    int nodes[4] = {0, 0, 0, 0};
+    double energy = 0.0;
+    bool lost = false;
+    if (ready && p < s.n) {
+      const int e = C.loc[threadIdx.x];
+      if (e >= 0)
+        push_fp64_one<AXI>(m, f, prm, s, p, e, C.x[threadIdx.x], C.y[threadIdx.x], C.vx[threadIdx.x],
+                           C.vy[threadIdx.x], key, W, nodes, energy, lost);
     }
-    if (in) {  // a dead or absent one of the two gets back what was read
-      if (prm.do_push) {
-        *reinterpret_cast<double2 *>(s.x + p) = *reinterpret_cast<const double2 *>(&C.x[q0]);
-        *reinterpret_cast<double2 *>(s.y + p) = *reinterpret_cast<const double2 *>(&C.y[q0]);
-        *reinterpret_cast<double2 *>(s.vx + p) = *reinterpret_cast<const double2 *>(&C.vx[q0]);
-        *reinterpret_cast<double2 *>(s.vy + p) = *reinterpret_cast<const double2 *>(&C.vy[q0]);
-      }
-      *reinterpret_cast<int2 *>(s.loc + p) = *reinterpret_cast<const int2 *>(&C.loc[q0]);
-    }
-    if (!prm.do_energy) {
-      if (lane == 0 && gone) atomicAdd(s.lost, (unsigned long long)gone);
-      if (prm.do_deposit) pair_deposit<!AXI>(m, s, lane, keys[0], qs[0], keys[1], qs[1]);
-    }
+    warp_deposit<!AXI>(s, lane, key, W, nodes, energy, lost, prm.do_deposit, prm.do_energy);
+    push_select_cta(s, key, p, pid, sel_buf);
     __syncthreads();  // tile t is read before its stage is refilled
   }
   push_select_flush(s, sel_buf);
@@ -3768,16 +3719,16 @@ static int run_push(int sidx, bool do_push, bool do_deposit, bool do_energy) {
   } else if (g.push64_grid > 0 && g.push64_bulk) {
     const int64_t ntiles = (s.n_slots + kPushTile - 1) / kPushTile;
     const unsigned grid = (unsigned)std::min<int64_t>(ntiles, g.push64_grid);
-    const size_t smem = kF64Stages * sizeof(PushTile64) + kF64Stages * sizeof(uint64_t);
+    const size_t smem = 3 * sizeof(PushTile64) + 3 * sizeof(uint64_t);
     if (g.axi)
-      k_push_bulk<kF64Stages, true><<<grid, kPairThreads, smem, g.st>>>(mesh_k(), f, prm, k, ntiles, g.push_wait_limit,
+      k_push_bulk<3, true><<<grid, kPushTile, smem, g.st>>>(mesh_k(), f, prm, k, ntiles, g.push_wait_limit,
                                                              g.push_skip_copies);
     else
       if (g.push64_minb == 5)
-        k_push_bulk<kF64Stages, false, 5><<<grid, kPairThreads, smem, g.st>>>(mesh_k(), f, prm, k, ntiles, g.push_wait_limit,
+        k_push_bulk<3, false, 5><<<grid, kPushTile, smem, g.st>>>(mesh_k(), f, prm, k, ntiles, g.push_wait_limit,
                                                                    g.push_skip_copies);
       else
-        k_push_bulk<kF64Stages, false><<<grid, kPairThreads, smem, g.st>>>(mesh_k(), f, prm, k, ntiles, g.push_wait_limit,
+        k_push_bulk<3, false><<<grid, kPushTile, smem, g.st>>>(mesh_k(), f, prm, k, ntiles, g.push_wait_limit,
                                                                 g.push_skip_copies);
   } else if (g.push64_grid > 0) {
     const int64_t ntiles = (s.n_slots + kPushTile - 1) / kPushTile;
@@ -5428,8 +5379,7 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     // FP64 push: particle tiles (9 KB each, 3 stages = 27 KB per CTA) staged
     // through shared memory when PIC_PUSH64_TILED is 1; otherwise one
     // particle per thread loaded directly (same bits either way)
-    // (2: bulk-copied by one thread, completing on mbarriers: kF64Stages tiles
-    // a CTA of kPairThreads threads, two particles a thread)
+    // (2: the tiles are bulk-copied by one thread and complete on mbarriers)
     // test hooks of the bulk-staged pushes' bounded wait: polls of a tile's
     // mbarrier before giving up, and no copies issued at all (every wait then
     // runs out and the step reports the failure)
@@ -5444,13 +5394,13 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     if (mode64 == 1 || mode64 == 2) {
       const char *m64 = getenv("PIC_PUSH64_MINB");  // 5: the Cartesian bulk push built for 5 CTAs per SM
       g.push64_minb = (m64 && atoi(m64) == 5 && !g.axi) ? 5 : 4;
-      const void *fn = g.push64_bulk ? (g.axi ? (const void *)k_push_bulk<kF64Stages, true>
-                                              : g.push64_minb == 5 ? (const void *)k_push_bulk<kF64Stages, false, 5>
-                                                                   : (const void *)k_push_bulk<kF64Stages, false>)
+      const void *fn = g.push64_bulk ? (g.axi ? (const void *)k_push_bulk<3, true>
+                                              : g.push64_minb == 5 ? (const void *)k_push_bulk<3, false, 5>
+                                                                   : (const void *)k_push_bulk<3, false>)
                                      : (g.axi ? (const void *)k_push_tiled<3, true> : (const void *)k_push_tiled<3, false>);
-      const size_t smem = g.push64_bulk ? kF64Stages * (sizeof(PushTile64) + sizeof(uint64_t)) : 3 * sizeof(PushTile64);
+      const size_t smem = 3 * sizeof(PushTile64) + (g.push64_bulk ? 3 * sizeof(uint64_t) : 0);
       int per_sm = 0;
-      PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, g.push64_bulk ? kPairThreads : kPushTile, smem));
+      PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kPushTile, smem));
       g.push64_grid = per_sm * nsm;
     }
   }
