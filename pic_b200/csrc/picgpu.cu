@@ -1188,7 +1188,8 @@ __global__ void __launch_bounds__(kPairThreads, MINB) k_push_mixed_bulk(MeshK m,
     if (s_fail) break;  // read after the CTA barrier that ends each tile: the same for every thread
     if (threadIdx.x == 0) {
       const int64_t tn = t + (S - 1) * G;
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      // the stage refilled here was left by every thread at the barrier that
+      // closed the previous tile, each behind its own proxy fence
       if (tn < ntiles && !skip_copies)
         push_tile_bulk(&T[(it + S - 1) % S], &bar[(it + S - 1) % S], s, tn * kPushTile);
     }
@@ -1255,7 +1256,10 @@ __global__ void __launch_bounds__(kPairThreads, MINB) k_push_mixed_bulk(MeshK m,
       if (lane == 0 && gone) atomicAdd(s.lost, (unsigned long long)gone);
       if (prm.do_deposit) pair_deposit<!AXI>(m, s, lane, keys[0], qs[0], keys[1], qs[1]);
     }
-    __syncthreads();  // tile t is read before its stage is refilled
+    // the tile was read and written with ordinary accesses: every thread orders
+    // its own before the bulk copy that refills the stage after the barrier
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncthreads();
   }
   push_select_flush(s, sel_buf);
 }

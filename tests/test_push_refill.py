@@ -16,7 +16,7 @@ SRC = os.path.join(os.path.dirname(api.__file__), "csrc", "picgpu.cu")
 FENCE = 'asm volatile("fence.proxy.async.shared::cta;\\n" ::: "memory");'
 
 
-@pytest.mark.parametrize("kernel", ["k_push_bulk"])
+@pytest.mark.parametrize("kernel", ["k_push_bulk", "k_push_mixed_bulk"])
 def test_stores_to_the_tile_are_fenced_by_every_thread(kernel):
     text = open(SRC).read()
     start = text.index("{", text.index(") " + kernel + "("))
@@ -35,7 +35,9 @@ def test_stores_to_the_tile_are_fenced_by_every_thread(kernel):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,prec,env", [("tiny", api.PIC_PREC_FP64, "PIC_PUSH64_TILED"),
-                                           ("tiny_axi", api.PIC_PREC_FP64, "PIC_PUSH64_TILED")])
+                                           ("tiny_axi", api.PIC_PREC_FP64, "PIC_PUSH64_TILED"),
+                                           ("tiny", api.PIC_PREC_MIXED, "PIC_PUSH_BULK"),
+                                           ("tiny_axi", api.PIC_PREC_MIXED, "PIC_PUSH_BULK")])
 def test_refilled_stages_match_single_particles(name, prec, env, monkeypatch):
     n = 2_500_001  # 9,766 tiles: several for each resident CTA, the last one of one particle
     got = {}
