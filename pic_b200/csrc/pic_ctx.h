@@ -196,6 +196,7 @@ struct Ctx {
   int push64_minb = 4;                      // resident CTAs per SM the Cartesian bulk push is built for
   bool push_bulk = false;                   // mixed-precision tiles bulk-copied (PIC_PUSH_BULK=1)
   int push_bulk_default = 1;
+  bool push_by_count = false;               // few particles: one a thread, loaded directly
   long long push_wait_limit = 1ll << 22;    // polls of a tile's mbarrier before the push gives up
   int push_skip_copies = 0;                 // test hook: the bulk pushes issue no tile copies
   // CUDA graphs of one FCG iteration: [0] stage A, [1 + slot] stage B + FCG

@@ -3683,9 +3683,19 @@ static int run_push(int sidx, bool do_push, bool do_deposit, bool do_energy) {
     pm.do_deposit = do_deposit;
     pm.do_energy = do_deposit && do_energy;
     for (int w = 0; w < 4; ++w) pm.wall[w] = g.P.wall_bc[w];
-    if (g.push_bulk && g.push_stages) {
-      // tiles bulk-copied by one thread (4 stages, 5 CTAs per SM)
-      const int64_t ntiles = (s.n_slots + kPushTile - 1) / kPushTile;
+    const int64_t ntiles = (s.n_slots + kPushTile - 1) / kPushTile;
+    // A tile or less for each resident CTA of the bulk form (1184 tiles,
+    // 303,104 slots on 148 SMs): its two particles a thread, one wave of half
+    // the warps, are slower than one each (us a launch at 20,000 / 85,000 /
+    // 254,000 particles: 10.8 / 10.8 / 12.8 against 7.9 / 8.3 / 11.6, r-z 11.8 /
+    // 12.8 / 14.9 against 8.7 / 9.7 / 14.1); with two tiles a CTA it is level
+    // (508,000: 17.6 against 18.1), and ahead beyond.  A form asked for by
+    // name runs at every count.
+    if (g.push_by_count && ntiles <= g.push_grid) {
+      if (g.axi) k_push_mixed<true><<<blocks_for(s.n_slots, 256), 256, 0, g.st>>>(m, g.d_coef32, pm, k);
+      else k_push_mixed<false><<<blocks_for(s.n_slots, 256), 256, 0, g.st>>>(m, g.d_coef32, pm, k);
+    } else if (g.push_bulk && g.push_stages) {
+      // tiles bulk-copied by one thread, two particles a thread
       const unsigned grid = (unsigned)std::min<int64_t>(ntiles, g.push_grid);
       const size_t smem = kMixStages * sizeof(PushTile) + kMixStages * sizeof(uint64_t);
       if (g.axi)
@@ -3697,14 +3707,12 @@ static int run_push(int sidx, bool do_push, bool do_deposit, bool do_energy) {
     } else if (g.axi) {
       // r-z: the default tiled form (4 stages, 5 CTAs per SM) or the direct one
       if (g.push_stages) {
-        const int64_t ntiles = (s.n_slots + kPushTile - 1) / kPushTile;
         const unsigned grid = (unsigned)std::min<int64_t>(ntiles, g.push_grid);
         k_push_mixed_tiled<4, 5, true><<<grid, kPushTile, 4 * sizeof(PushTile), g.st>>>(m, g.d_coef32, pm, k, ntiles);
       } else {
         k_push_mixed<true><<<blocks_for(s.n_slots, 256), 256, 0, g.st>>>(m, g.d_coef32, pm, k);
       }
     } else if (g.push_stages) {
-      const int64_t ntiles = (s.n_slots + kPushTile - 1) / kPushTile;
       const unsigned grid = (unsigned)std::min<int64_t>(ntiles, g.push_grid);
       const size_t smem = (size_t)g.push_stages * sizeof(PushTile);
       if (g.push_stages == 2)
@@ -5391,6 +5399,9 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     if (wl && atoll(wl) > 0) g.push_wait_limit = atoll(wl);
     const char *sc = getenv("PIC_PUSH_SKIP_COPIES");
     g.push_skip_copies = sc && atoi(sc) == 1 ? 1 : 0;
+    // the mixed push chooses its form by the particle count unless one was named
+    g.push_by_count = g.push_bulk && !g.push_skip_copies && !getenv("PIC_PUSH_BULK") && !getenv("PIC_PUSH_STAGES") &&
+                      !getenv("PIC_PUSH_MINB");
     const char *p64 = getenv("PIC_PUSH64_TILED");
     const int mode64 = p64 ? atoi(p64) : g.push64_default;
     g.push64_grid = 0;
