@@ -17,7 +17,7 @@ __device__ __forceinline__ double div_const(double a, double d, double y, bool &
   q = fma(fma(-q, d, a), y, q);
   q = fma(fma(-q, d, a), y, q);
   const double m = fabs(a);
-  exact = exact && ((m > 1e-250 && m < 1e250 && y == y) || m == 0.0);
+  exact = exact && y == y && ((m > 1e-250 && m < 1e250) || m == 0.0);
   return m == 0.0 ? zero : q;
 }
 
@@ -26,9 +26,13 @@ __device__ __forceinline__ double recip_const(double d) {
   return m > 1e-40 && m < 1e40 ? 1.0 / d : __longlong_as_double(0x7ff8000000000000ll);
 }
 
-// 1/d rounded to nearest, from y0 = 1/d0 of a divisor d0 that d equals to
-// about 1e-9 (NaN stays NaN): one Newton step brings it to within its last
-// place, and the next rounds correctly (Markstein's theorem for reciprocals).
+// 1/d from y0 = 1/d0 of a divisor d0 that d equals to about 1e-9 (NaN stays
+// NaN): one Newton step brings it to within its last place, and the next rounds
+// correctly by Markstein's theorem for reciprocals, but for a significand of
+// all ones (its exception), where y may be the power of two just below.  Then
+// too div_const's quotients are right: y d = 1 - 2^-53, so the last correction
+// is off by 2^-53 of half a unit, and no quotient by such a d lies that near to
+// a midpoint but a power of two's, which comes out above it, as it is.
 __device__ __forceinline__ double recip_near(double d, double y0) {
   const double y = fma(fma(-d, y0, 1.0), y0, y0);
   return fma(fma(-d, y, 1.0), y, y);
