@@ -26,16 +26,16 @@ __device__ __forceinline__ double recip_const(double d) {
   return m > 1e-40 && m < 1e40 ? 1.0 / d : __longlong_as_double(0x7ff8000000000000ll);
 }
 
-// 1/d from y0 = 1/d0 of a divisor d0 that d equals to about 1e-9 (NaN stays
-// NaN): one Newton step brings it to within its last place, and the next rounds
-// correctly by Markstein's theorem for reciprocals, but for a significand of
-// all ones (its exception), where y may be the power of two just below.  Then
-// too div_const's quotients are right: y d = 1 - 2^-53, so the last correction
-// is off by 2^-53 of half a unit, and no quotient by such a d lies that near to
-// a midpoint but a power of two's, which comes out above it, as it is.
+// 1/d rounded to nearest, from y0 = 1/d0 of a divisor d0 that d equals to
+// about 1e-9 (NaN stays NaN): one Newton step brings it to within its last
+// place, and the next rounds correctly (Markstein's theorem for reciprocals).
+// The theorem leaves out a significand of all ones, where y can stay a place
+// low and the quotient of a power of two with it: NaN there, so the caller divides.
 __device__ __forceinline__ double recip_near(double d, double y0) {
-  const double y = fma(fma(-d, y0, 1.0), y0, y0);
-  return fma(fma(-d, y, 1.0), y, y);
+  const long long ones = (1ll << 52) - 1;
+  double y = fma(fma(-d, y0, 1.0), y0, y0);
+  y = fma(fma(-d, y, 1.0), y, y);
+  return (__double_as_longlong(d) & ones) == ones ? __longlong_as_double(0x7ff8000000000000ll) : y;
 }
 
 }  // namespace pic

@@ -3,6 +3,7 @@ range, a zero numerator among them: the division is taken."""
 import numpy as np
 import pytest
 
+from test_noalloc_runs import _law
 from pic_b200 import api, deck, simulation
 
 pytestmark = pytest.mark.gpu
@@ -30,6 +31,34 @@ def test_deposit_on_meshes_of_any_scale(h):
     want[0, :2] += 0.5                      # (0, h): the cells are 2h tall
     # positions are within an ulp or two of the nodes, charges within 2^-40
     assert np.abs(out.cpu().numpy().reshape(nnx, nny) - want).max() < 1e-11
+
+
+@pytest.mark.parametrize("quarters,steps", [(3, 0), (4, -1), (13, -1), (27, 0)])
+def test_deposit_in_cells_a_unit_short_of_a_power_of_two(quarters, steps):
+    """xmin off zero by a few quarters of 2^-53: the first cell's width rounds
+    to 1 - 2^-53, the divisor whose reciprocal Newton's steps leave a place low."""
+    import torch
+    lib = api.load()
+    nnx, nny = 3, 4
+    xmin = 0.0625 + quarters * 2.0 ** -55
+    xmax = xmin + 2.0
+    for _ in range(-steps):
+        xmax = np.nextafter(xmax, 0.0)
+    assert (xmin + (xmax - xmin) / 2) - xmin == 1.0 - 2.0 ** -53
+    # a power of two into the cell; (1 - dy) dx 2^40 on one side of k + 1/2, by
+    # the last place of dx
+    k = np.arange(0, 64, 2)
+    y = 1.0 - (2.0 * k + 1.0) * 2.0 ** -37
+    x = np.full(y.size, xmin + 0.0625)
+    assert np.all(x - xmin == 0.0625)
+    n, vol, loc = x.size, np.ones(nnx * nny), np.zeros(x.size, np.int32)
+    t = [torch.from_numpy(a).cuda() for a in (x, y, vol)]
+    out = torch.zeros(nnx * nny, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    api.check(lib.pic_deposit_noalloc(nnx, nny, xmin, xmax, 0.0, nny - 1.0, n, t[0].data_ptr(), t[1].data_ptr(), None,
+                                      t[2].data_ptr(), 1.0, 1.0, 1.0, out.data_ptr(), None), "pic_deposit_noalloc")
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy(), _law(nnx, nny, xmin, xmax, 0.0, nny - 1.0, x, y, loc, vol, 1.0, 1.0, 1.0))
 
 
 @pytest.mark.parametrize("scale", [2.0 ** -150, 2.0 ** -136, 2.0 ** 140])
