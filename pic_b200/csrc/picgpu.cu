@@ -2162,6 +2162,9 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
   __syncthreads();
   double rho = __ldcg(&S->rho);
   const double normRHS = __ldcg(&S->normRHS), tol2 = S->tol2;
+  // a residual beyond this is far from converged; always the quotient where it
+  // or the bound could underflow
+  const double far = tol2 > 1e-290 && tol2 * normRHS > 1e-290 ? 2.0 * tol2 * normRHS : (double)INFINITY;
   const int maxit = S->maxit;
   int done = __ldcg(&S->done), iter = 0, ierr = 0;
   double beta = 0.0, normR = 0.0, rho0 = 0.0;
@@ -2317,7 +2320,7 @@ __global__ void __launch_bounds__(256 * NG, 1) k_pcg_smem(PcgS P) {
     rho = tot[1];
     ++iter;
     // the division only where the comparison could turn on its rounding
-    if (!(normR > 2.0 * tol2 * normRHS) && normR / normRHS <= tol2) done = 1;
+    if (!(normR > far) && normR / normRHS <= tol2) done = 1;
     else if (iter >= maxit) { ierr = 1; done = 1; }
     else if (rho0 == 0.0) { ierr = 2; done = 1; }
     else beta = rho / rho0;
