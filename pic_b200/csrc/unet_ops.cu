@@ -508,7 +508,8 @@ __device__ __forceinline__ void wg_stage(WgTile<MT> &T, int tile, int ti, int tj
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-template <int MT>
+// RAGGED: tiles may reach past the image (its tests: 2% of a training step)
+template <int MT, bool RAGGED>
 __global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, int c, int k, const bf16 *__restrict__ x,
                                                           const bf16 *__restrict__ dy, float *__restrict__ dw) {
   extern __shared__ __align__(128) unsigned char wg_smem[];
@@ -537,7 +538,13 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, i
     }
     __syncthreads();
     const WgTile<MT> &S = T[stage];
-    for (int row = 0; row < WG_ROWS; ++row) {
+    // Past the image's last row and column dy is zero-filled, and taps that reach
+    // back inside would multiply real activations by those zeros (an infinite
+    // one to NaN): rows past the end are left out, and so is the one column
+    // that reaches back, at the first column's taps
+    const int rows = RAGGED ? min(WG_ROWS, h - tile / tj % ti * WG_ROWS) : WG_ROWS;
+    const int past = RAGGED && ts == 0 ? w - tile % tj * WG_PIX : WG_PIX;  // WG_PIX or more: none
+    for (int row = 0; row < rows; ++row) {
       unsigned A[2][MT][4], B[2][2][4];
 #pragma unroll
       for (int s = 0; s < 2; ++s) {  // 16 pixels of the row each
@@ -546,6 +553,16 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, i
 #pragma unroll
         for (int q = 0; q < 2; ++q)
           wg_ldsm4t(B[s][q], &S.x[(row + tr) * (WG_PIX + 2) + 16 * s + ts + bpix][16 * q + bch]);
+      }
+      if (past < WG_PIX && (past & 7) >> 1 == (lane & 3)) {  // a lane holds two pixels of every eight
+        const unsigned keep = past & 1 ? 0x0000ffffu : 0xffff0000u;
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (past >> 3 == 2 * s + (e & 1)) B[s][q][e] &= keep;
       }
 #pragma unroll
       for (int a = 0; a < MT; ++a)
@@ -579,14 +596,15 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, i
 template <int MT>
 int run_wgrad_mma(int n, int h, int w, int c, int k, const bf16 *x, const bf16 *dy, float *dw, cudaStream_t st) {
   const size_t smem = 2 * sizeof(WgTile<MT>);
+  const auto fn = h % WG_ROWS || w % WG_PIX ? k_wgrad_mma<MT, true> : k_wgrad_mma<MT, false>;
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k_wgrad_mma<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return UNET_ERR_CUDA;
   const unsigned gx = (unsigned)(((k + 16 * MT - 1) / (16 * MT)) * ((c + 31) / 32));
   const int64_t tiles = (int64_t)n * ((h + WG_ROWS - 1) / WG_ROWS) * ((w + WG_PIX - 1) / WG_PIX);
   int64_t gy = (2 * 148 + gx - 1) / gx;
   if (gy > (tiles + 1) / 2) gy = (tiles + 1) / 2;
-  k_wgrad_mma<MT><<<dim3(gx, (unsigned)gy), WG_THREADS, smem, st>>>(n, h, w, c, k, x, dy, dw);
+  fn<<<dim3(gx, (unsigned)gy), WG_THREADS, smem, st>>>(n, h, w, c, k, x, dy, dw);
   return launched();
 }
 

@@ -1,0 +1,54 @@
+"""The tensor-core weight gradient beside the image's ends: an infinite
+activation reaches the taps that pair it with a pixel of the image and no
+others (tiles of 4 rows x 32 pixels, the rest of them zero-filled)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def P(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _law(x, dy):
+    """[k, 3, 3, c] in FP64: sums over the pairs inside the image only."""
+    n, h, w, c = x.shape
+    out = torch.zeros(dy.shape[3], 3, 3, c, dtype=torch.float64)
+    for r in range(3):
+        for s in range(3):
+            i0, i1, j0, j1 = max(0, 1 - r), min(h, h + 1 - r), max(0, 1 - s), min(w, w + 1 - s)
+            d = dy[:, i0:i1, j0:j1].reshape(-1, dy.shape[3]).double()
+            v = x[:, i0 + r - 1:i1 + r - 1, j0 + s - 1:j1 + s - 1].reshape(-1, c).double()
+            out[:, r, s] = (d[:, :, None] * v[:, None, :]).sum(0)
+    return out
+
+
+@pytest.mark.parametrize("where", ["last column", "last row", "corner"])
+@pytest.mark.parametrize("h,w", [(4, 32), (5, 33), (6, 63), (7, 40), (3, 31), (2, 1), (1, 18), (8, 47)])
+@pytest.mark.parametrize("c,k", [(8, 32), (40, 64)])
+def test_infinite_activations_stay_in_their_taps(c, k, h, w, where):
+    from pic_b200 import unet
+    lib = unet.load()
+    g = torch.Generator().manual_seed(100 * h + w)
+    x = torch.randn(2, h, w, c, generator=g).bfloat16()
+    dy = (torch.rand(2, h, w, k, generator=g) + 0.5).bfloat16()  # one sign: no inf - inf
+    if where == "last column":
+        x[:, :, w - 1, 3] = float("inf")
+    elif where == "last row":
+        x[:, h - 1, :, 5] = float("inf")
+    else:
+        x[1, h - 1, w - 1, :] = float("inf")
+    dw = torch.zeros(k, 3, 3, c, dtype=torch.float32, device="cuda")
+    xd, dyd = x.cuda(), dy.cuda()
+    assert lib.unet_wgrad(2, h, w, c, k, P(xd), P(dyd), P(dw), None) == 0
+    torch.cuda.synchronize()
+    got, want = dw.double().cpu(), _law(x, dy)
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), finite)
+    assert torch.equal(got[~finite], want[~finite])
+    # FP32 sums of up to 750 exact products
+    assert (got[finite] - want[finite]).abs().max() <= 1e-5 * max(1.0, float(want[finite].abs().max())) if finite.any() else True
