@@ -515,7 +515,9 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, i
   extern __shared__ __align__(128) unsigned char wg_smem[];
   WgTile<MT> *T = reinterpret_cast<WgTile<MT> *>(wg_smem);
   const int ncb = (c + 31) / 32, kb = blockIdx.x / ncb, cb = blockIdx.x % ncb;
-  const int ti = (h + WG_ROWS - 1) / WG_ROWS, tj = (w + WG_PIX - 1) / WG_PIX, tiles = n * ti * tj;
+  const int ti = (h + WG_ROWS - 1) / WG_ROWS, tj = (w + WG_PIX - 1) / WG_PIX;
+  // up to 2^31 - 1 tiles (images of one pixel): the step past the last one still fits
+  const unsigned tiles = (unsigned)(n * ti * tj);
   const int lane = threadIdx.x & 31, tap = threadIdx.x >> 5, tr = tap / 3, ts = tap % 3;
   float acc[MT][4][4];
 #pragma unroll
@@ -527,11 +529,12 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_mma(int n, int h, int w, i
   const int apix = (lane & 7) + ((lane >> 4) & 1) * 8, ach = ((lane >> 3) & 1) * 8;
   const int bpix = (lane & 7) + ((lane >> 3) & 1) * 8, bch = ((lane >> 4) & 1) * 8;
   int stage = 0;
-  if ((int)blockIdx.y < tiles) wg_stage<MT>(T[0], blockIdx.y, ti, tj, h, w, c, k, kb, cb, x, dy);
-  for (int tile = blockIdx.y; tile < tiles; tile += gridDim.y, stage ^= 1) {
-    const int next = tile + gridDim.y;
+  if (blockIdx.y < tiles) wg_stage<MT>(T[0], (int)blockIdx.y, ti, tj, h, w, c, k, kb, cb, x, dy);
+  for (unsigned at = blockIdx.y; at < tiles; at += gridDim.y, stage ^= 1) {
+    const int tile = (int)at;
+    const unsigned next = at + gridDim.y;
     if (next < tiles) {
-      wg_stage<MT>(T[stage ^ 1], next, ti, tj, h, w, c, k, kb, cb, x, dy);
+      wg_stage<MT>(T[stage ^ 1], (int)next, ti, tj, h, w, c, k, kb, cb, x, dy);
       asm volatile("cp.async.wait_group 1;" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;" ::: "memory");

@@ -2,12 +2,12 @@
 activation reaches the taps that pair it with a pixel of the image and no
 others (tiles of 4 rows x 32 pixels, the rest of them zero-filled)."""
 import ctypes as C
+import os
+import re
 
-import numpy as np
 import pytest
 
 torch = pytest.importorskip("torch")
-pytestmark = pytest.mark.gpu
 
 
 def P(t):
@@ -27,6 +27,7 @@ def _law(x, dy):
     return out
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("where", ["last column", "last row", "corner"])
 @pytest.mark.parametrize("h,w", [(4, 32), (5, 33), (6, 63), (7, 40), (3, 31), (2, 1), (1, 18), (8, 47)])
 @pytest.mark.parametrize("c,k", [(8, 32), (40, 64)])
@@ -52,3 +53,17 @@ def test_infinite_activations_stay_in_their_taps(c, k, h, w, where):
     assert torch.equal(got[~finite], want[~finite])
     # FP32 sums of up to 750 exact products
     assert (got[finite] - want[finite]).abs().max() <= 1e-5 * max(1.0, float(want[finite].abs().max())) if finite.any() else True
+
+
+def test_tile_counter_does_not_wrap():
+    """Up to 2^31 - 1 tiles go to the kernel, and its CTAs step past the last one
+    by up to their number: counted in 32 bits without a sign (34 GB operands:
+    read from the source)."""
+    from pic_b200 import unet
+    src = open(os.path.join(os.path.dirname(unet.__file__), "csrc", "unet_ops.cu")).read()
+    body = src[src.index(") k_wgrad_mma("):src.index("int run_wgrad_mma(")]
+    loop = re.search(r"for \((\w+) (\w+) = blockIdx\.y; \2 < tiles; \2 \+= gridDim\.y", body)
+    assert loop and loop.group(1) == "unsigned"
+    assert re.search(r"const unsigned next = %s \+ gridDim\.y;" % loop.group(2), body)
+    assert re.search(r"const unsigned tiles = ", body)
+    assert "np < ((int64_t)1 << 31)" in src[src.index("int unet_wgrad("):]
