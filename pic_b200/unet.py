@@ -116,7 +116,7 @@ class ParamSet(dict):
         for name, t in values.items():
             at[name] = total
             total += -(-t.numel() // self.ALIGN) * self.ALIGN
-        host = torch.zeros(total)
+        host = torch.zeros(total, dtype=torch.float32)  # whatever the default type
         for name, t in values.items():
             host[at[name]:at[name] + t.numel()] = t.reshape(-1)
         p = host.to("cuda")
