@@ -5289,8 +5289,13 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     per_sm_f = std::min(per_sm_f, per_sm_f32);
     const char *envf = getenv("PIC_FCG_PERSISTENT");
     const bool want_f = !(envf && envf[0] == '0');
-    g.fcg_coop_grid =
-        (want_f && coop && per_sm_f > 0 && nn < kMarchMaxNodes) ? std::min(g.red_blocks, nsm) : 0;
+    // a CTA for every kFcgT nodes while the SMs last, two at least (of each
+    // chunk, so d_fcg_part holds 4 of the grid's partials): with one for every
+    // chunk, half the threads of the solve shared the dense coarse inverse
+    // (64^2, two-level: 0.785 -> 0.502 ms; 96^2 V-cycle 0.441 -> 0.319)
+    g.fcg_coop_grid = (want_f && coop && per_sm_f > 0 && nn < kMarchMaxNodes)
+                          ? (int)std::min<int64_t>(std::max<int64_t>((nn + kFcgT - 1) / kFcgT, 2), nsm)
+                          : 0;
     // the explicit rows of each CTA's columns, for its shared-memory table
     if (g.fcg_coop_grid > 0 && g.ex_stencil) {
       std::vector<int2> kr(g.fcg_coop_grid);

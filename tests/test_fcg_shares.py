@@ -1,0 +1,67 @@
+"""The persistent flexible CG hands out its nodes so that no CTA, and no half of
+one, idles: grids of few nodes, grids with fewer columns than CTAs.  Against the
+launch-per-operation path (which sums dot products in another order: the same
+iterations within 2 and potentials within 1e-7, the bars of the multigrid
+tests), and by time against a grid that has no such shortage."""
+import numpy as np
+import pytest
+
+from pic_b200 import api, deck
+from pic_b200.simulation import Simulation
+
+pytestmark = pytest.mark.gpu
+
+
+def _sim(name, ncx, ncy, walls=(1, 1, 1, 1), tol=1e-10, **solver):
+    h = 0.01 / 16
+    R = min(ncx, ncy) * h
+    obj = deck.ObjectSpec(api.PIC_SHAPE_CIRCLE, 0.5013 * ncx * h, 0.5471 * ncy * h, 0.2137 * R, eps=4.0)
+    cfg = deck.config(name, ncx=ncx, ncy=ncy, Lx=ncx * h, Ly=ncy * h, objects=[obj], wall_dirichlet=walls, pcg_tol=tol)
+    sim = Simulation(cfg, load=False, capacity=[16, 16], mcc=False)
+    sim.set_solver("fcg", window=1, omega=0.8, **solver)
+    sim.set_field("rho", 0.05 * np.random.default_rng(ncx + ncy).standard_normal((ncx + 1) * (ncy + 1)))
+    return sim
+
+
+def _best_ms(ncx, ncy):
+    sim = _sim("tiny", ncx, ncy, multigrid=True)
+    try:
+        best = 1e9
+        for _ in range(12):
+            sim.set_field("phi", sim.mesh.array("phi_dirichlet"))
+            best = min(best, sim.ife_solve().ms)
+        return best
+    finally:
+        sim.close()
+
+
+# one CTA; more CTAs than columns; a last block of rows left to single nodes
+@pytest.mark.parametrize("name,ncx,ncy,walls,solver", [
+    ("tiny", 16, 16, (1, 1, 1, 1), {"coarse_cells": 8}), ("tiny", 32, 16, (1, 1, 1, 1), {"coarse_cells": 8}),
+    ("tiny", 8, 512, (1, 1, 1, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
+    ("tiny", 8, 1600, (1, 0, 0, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
+    ("tiny_axi", 16, 800, (0, 1, 0, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
+    ("tiny", 48, 96, (1, 1, 1, 1), {"multigrid": True, "max_coarse_nodes": 1300})])
+def test_shares_match_the_launched_kernels(name, ncx, ncy, walls, solver, monkeypatch):
+    got = {}
+    for mode in ("1", "0"):
+        monkeypatch.setenv("PIC_FCG_PERSISTENT", mode)
+        sim = _sim(name, ncx, ncy, walls, **dict(solver))
+        try:
+            phi = sim.mesh.array("phi_dirichlet").copy()
+            st = sim.ife_solve(phi)
+            assert st.ierr == 0 and st.fallback == 0
+            got[mode] = (st.iterations, phi)
+        finally:
+            sim.close()
+    assert abs(got["1"][0] - got["0"][0]) <= 2
+    assert np.abs(got["1"][1] - got["0"][1]).max() <= 1e-7 * np.abs(got["0"][1]).max()
+
+
+def test_one_kernel_beats_the_launched_ones_on_a_small_grid(monkeypatch):
+    t = {}
+    for mode in ("1", "0"):
+        monkeypatch.setenv("PIC_FCG_PERSISTENT", mode)
+        t[mode] = _best_ms(128, 128)
+    # 0.73 of their time; with a CTA of 512 threads for every 1024 nodes 1.07
+    assert t["1"] <= 0.9 * t["0"]
