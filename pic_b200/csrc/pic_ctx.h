@@ -160,6 +160,7 @@ struct Ctx {
   int red_blocks = 0;
   int coop_grid = 0;               // CTAs of the persistent PCG (0: two-kernel loop)
   int fcg_coop_grid = 0;           // CTAs of the persistent FCG (0: graph-launched iterations)
+  int fcg_band_blocks = 0;         // row blocks of a band of its column walk
   int smem_grid = 0, smem_cpc = 0; // CTAs of the on-chip PCG (0: not eligible) and their chunks at most
   ulonglong2 *d_pcg_slot = nullptr, *d_pcg_strip = nullptr;  // its tagged partials and boundary strips
   unsigned pcg_tag = 1;            // the next solve's first tag

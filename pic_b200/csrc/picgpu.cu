@@ -2737,6 +2737,7 @@ struct FcgP {
   int ainv_stream;               // the vectors fill L2: read the inverse past it
   double *rc, *ec;
   int nnx, cs, ncx, ncy, coarse;
+  int band_blocks;               // row blocks of a band of the column walk (fcg_share)
   MgK mg;                        // multigrid V-cycle (mg.L > 1) in place of the two-level space
   double omega;
   const int2 *tab_rows;          // per CTA: first kind and count of its explicit rows in shared memory (or null)
@@ -2909,6 +2910,57 @@ __device__ __forceinline__ V stencil9(const PcgK &k, const StTab &tab, int kind,
 // 2 x 512 + 1 rows is the common grid) is done node by node: rest(n).
 constexpr int kMarchRest = 64;
 
+// Rows of a block: a power of two where little is left over (513 = 512 + 1:
+// two groups of columns), so that no half of the CTA idles.
+__host__ __device__ inline int march_block(int nny) {
+  int blk = kFcgT;
+  while (blk > 64 && blk > nny) blk >>= 1;
+  return nny < kFcgT && nny - blk > kMarchRest ? nny : blk;
+}
+
+// Blocks of a column walk (a last one of at most kMarchRest rows goes with the
+// one before it).
+__host__ __device__ inline int march_blocks(int nny) {
+  const int blk = march_block(nny), rest = nny % blk;
+  return nny / blk + (rest > kMarchRest || nny < blk ? 1 : 0);
+}
+
+// CTA b's part of the fine grid: its columns [i0, i1) in its band's rows
+// [j0, j1).  One band of all rows mostly; grids with few columns have bands of
+// band_blocks row blocks (fcg_band_blocks), each for an equal group of CTAs.
+struct FcgShare {
+  int i0, i1, j0, j1;
+};
+
+__host__ __device__ inline FcgShare fcg_share(int b, int G, int nnx, int nny, int band_blocks) {
+  const int blocks = march_blocks(nny), bands = (blocks + band_blocks - 1) / band_blocks;
+  const int per = G / bands, band = b / per, c = b - band * per;
+  if (band >= bands) return {0, 0, 0, 0};
+  const int rows = band_blocks * march_block(nny);
+  return {(int)((int64_t)c * nnx / per), (int)((int64_t)(c + 1) * nnx / per), band * rows,
+          band == bands - 1 ? nny : (band + 1) * rows};
+}
+
+// Bands for a grid with fewer than twice as many columns as CTAs: a walk costs
+// about its columns and the two beside them, for every block of rows, and one
+// band leaves CTAs without a column.  64 x 8192 cells in one band kept 65 of
+// 148 CTAs busy, each with 16 blocks: 0.95 -> 0.53 ms a solve call (8192 x 64:
+// 0.58), 32 x 16384 1.53 -> 0.55, 256 x 2048 0.64 -> 0.56.
+inline int fcg_band_blocks(int G, int nnx, int nny) {
+  const int blocks = march_blocks(nny);
+  int best = blocks;
+  int64_t least = -1;
+  for (int bands = 1; bands <= std::min(blocks, nnx < 2 * G ? G : 1); ++bands) {
+    const int bb = (blocks + bands - 1) / bands, used = (blocks + bb - 1) / bb, per = G / used;
+    const int64_t cost = (int64_t)((nnx + per - 1) / per + 2) * bb;
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = bb;
+    }
+  }
+  return best;
+}
+
 // element m of an array through a 32-bit byte offset: one register for all
 // arrays of a phase (the solver takes at most kMarchMaxNodes nodes)
 constexpr int64_t kMarchMaxNodes = (int64_t)1 << 29;
@@ -2918,16 +2970,12 @@ __device__ __forceinline__ T &at(T *p, unsigned m) {
 }
 
 template <class V, class Load, class Eval, class Pre, class Body, class Rest>
-__device__ __forceinline__ void march(int nnx, int nny, int i0, int i1, Load load, Eval eval, Pre pre, Body body,
+__device__ __forceinline__ void march(int nnx, int nny, const FcgShare &S, Load load, Eval eval, Pre pre, Body body,
                                       Rest rest) {
-  const int lane = threadIdx.x & 31;
-  // rows of a block: a power of two where little is left over (513 = 512 + 1:
-  // two groups of columns), so that no half of the CTA idles
-  int blk = kFcgT;
-  while (blk > 64 && blk > nny) blk >>= 1;
-  if (nny < kFcgT && nny - blk > kMarchRest) blk = nny;
-  for (int jb = 0; jb < nny; jb += blk) {
-    const int rows = min(blk, nny - jb);
+  const int lane = threadIdx.x & 31, i0 = S.i0, i1 = S.i1;
+  const int blk = march_block(nny);
+  for (int jb = S.j0; jb < S.j1; jb += blk) {
+    const int rows = min(blk, S.j1 - jb);
     if (jb > 0 && rows <= kMarchRest) {
       for (int q = threadIdx.x; q < rows * (i1 - i0); q += kFcgT)
         rest((i0 + q / rows) * nny + jb + q % rows);
@@ -3015,7 +3063,9 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
   const int nc = F.ncx * F.ncy;
   // the CTA's own columns (explicit rows as lists: its nodes), contiguous: a
   // stencil's neighbour columns are mostly the CTA's own nodes too
-  const int i0 = (int)((int64_t)blockIdx.x * F.nnx / G), i1 = (int)((int64_t)(blockIdx.x + 1) * F.nnx / G);
+  __shared__ FcgShare own;  // (registers are short)
+  if (threadIdx.x == 0) own = fcg_share(blockIdx.x, G, F.nnx, k.nny, F.band_blocks);
+  __syncthreads();
   const int64_t n0 = (int64_t)blockIdx.x * nn / G, n1 = (int64_t)(blockIdx.x + 1) * nn / G;
   StTab tab{fcg_smem + F.ainv_ld, 0, 0};
   if (EX == 1 && sizeof(V) == sizeof(double) && F.tab_rows != nullptr) {
@@ -3067,7 +3117,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
         struct Raw { V r, q, d; };
         struct Pre { V x, p; int kind; };
         march<V>(
-            F.nnx, k.nny, i0, i1,
+            F.nnx, k.nny, own,
             [&](unsigned m, int, int) { return Raw{at(r, m), upd ? at(Qp, m) : (V)0, at(F.dinv, m)}; },
             [&](const Raw &v) { return (om * (upd ? vfma(-a, v.q, v.r) : v.r)) * v.d; },
             [&](unsigned n) { return Pre{upd ? at(F.x, n) : (V)0, upd ? at(Pl, n) : (V)0, at(k.row_kind, n)}; },
@@ -3222,7 +3272,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
         };
         auto eval = [&](const Raw &v) { return v.kind < 0 ? (V)0 : mgrid ? (V)((double)v.z + v.pe) : v.z; };
         march<V>(
-            F.nnx, k.nny, i0, i1, load, eval,
+            F.nnx, k.nny, own, load, eval,
             [&](unsigned n) { return Pre{at(F.dinv, n), at(r, n), have_old ? at(Ql, n) : (V)0}; },
             [&](unsigned n, const V(&w)[3][3], const Raw &v, const Pre &p) {
               put_e(n, v.kind < 0 ? (V)0 : vfma(om * p.d, p.r - stencil9<V>(k, tab, v.kind, w), w[1][1]), p.q);
@@ -3274,7 +3324,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
         struct Raw { V z, p; };
         struct Pre { V r; int kind; };
         march<V>(
-            F.nnx, k.nny, i0, i1,
+            F.nnx, k.nny, own,
             [&](unsigned m, int, int) { return Raw{at(F.zF, m), ho ? at(Pl, m) : (V)0}; },
             [&](const Raw &v) { return ho ? vfma(bt, v.p, v.z) : v.z; },
             [&](unsigned n) { return Pre{at(r, n), at(k.row_kind, n)}; },
@@ -4175,6 +4225,7 @@ static int run_fcg_persist64(pic_solve_stats *stats, int *fcg_iters, int *rc_out
   F.rc = g.d_pc_rc;
   F.ec = g.d_pc_ec;
   F.nnx = g.m.nnx;
+  F.band_blocks = g.fcg_band_blocks;
   F.cs = g.pc_cs;
   F.ncx = g.pc_ncx;
   F.ncy = g.pc_ncy;
@@ -4317,6 +4368,7 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
       F.rc = g.d_pc_rc;
       F.ec = g.d_pc_ec;
       F.nnx = g.m.nnx;
+      F.band_blocks = g.fcg_band_blocks;
       F.cs = g.pc_cs;
       F.ncx = g.pc_ncx;
       F.ncy = g.pc_ncy;
@@ -5296,19 +5348,20 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     g.fcg_coop_grid = (want_f && coop && per_sm_f > 0 && nn < kMarchMaxNodes)
                           ? (int)std::min<int64_t>(std::max<int64_t>((nn + kFcgT - 1) / kFcgT, 2), nsm)
                           : 0;
+    g.fcg_band_blocks = g.fcg_coop_grid > 0 ? fcg_band_blocks(g.fcg_coop_grid, m.nnx, m.nny) : 0;
     // the explicit rows of each CTA's columns, for its shared-memory table
     if (g.fcg_coop_grid > 0 && g.ex_stencil) {
       std::vector<int2> kr(g.fcg_coop_grid);
       int most = 0;
       for (int b = 0; b < g.fcg_coop_grid; ++b) {
-        const int64_t a0 = (int64_t)b * m.nnx / g.fcg_coop_grid * m.nny;
-        const int64_t a1 = (int64_t)(b + 1) * m.nnx / g.fcg_coop_grid * m.nny;
+        const FcgShare own = fcg_share(b, g.fcg_coop_grid, m.nnx, m.nny, g.fcg_band_blocks);
         int lo = INT_MAX, hi = -1;
-        for (int64_t n = a0; n < a1; ++n)
-          if (row_kind[n] >= g.n_mat) {
-            lo = std::min(lo, row_kind[n]);
-            hi = std::max(hi, row_kind[n]);
-          }
+        for (int i = own.i0; i < own.i1; ++i)
+          for (int64_t n = (int64_t)i * m.nny + own.j0; n < (int64_t)i * m.nny + own.j1; ++n)
+            if (row_kind[n] >= g.n_mat) {
+              lo = std::min(lo, row_kind[n]);
+              hi = std::max(hi, row_kind[n]);
+            }
         kr[b] = hi < 0 ? make_int2(0, 0) : make_int2(lo, hi - lo + 1);
         kr[b].y = std::min(kr[b].y, kFcgTabRows);  // the others come from global memory
         most = std::max(most, kr[b].y);

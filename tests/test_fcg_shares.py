@@ -35,11 +35,16 @@ def _best_ms(ncx, ncy):
         sim.close()
 
 
-# one CTA; more CTAs than columns; a last block of rows left to single nodes
+# two CTAs; more CTAs than columns; a last block of rows left to single nodes;
+# bands of row blocks, the last of 65 rows and of 512 + 1
 @pytest.mark.parametrize("name,ncx,ncy,walls,solver", [
     ("tiny", 16, 16, (1, 1, 1, 1), {"coarse_cells": 8}), ("tiny", 32, 16, (1, 1, 1, 1), {"coarse_cells": 8}),
     ("tiny", 8, 512, (1, 1, 1, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
     ("tiny", 8, 1600, (1, 0, 0, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
+    ("tiny", 8, 2048, (0, 1, 1, 0), {"multigrid": True, "max_coarse_nodes": 1200}),
+    ("tiny", 64, 1024, (1, 1, 1, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
+    ("tiny", 8, 4160, (1, 1, 1, 1), {"multigrid": True, "max_coarse_nodes": 5000}),
+    ("tiny_axi", 16, 4096, (0, 1, 0, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
     ("tiny_axi", 16, 800, (0, 1, 0, 1), {"multigrid": True, "max_coarse_nodes": 1200}),
     ("tiny", 48, 96, (1, 1, 1, 1), {"multigrid": True, "max_coarse_nodes": 1300})])
 def test_shares_match_the_launched_kernels(name, ncx, ncy, walls, solver, monkeypatch):
@@ -65,3 +70,8 @@ def test_one_kernel_beats_the_launched_ones_on_a_small_grid(monkeypatch):
         t[mode] = _best_ms(128, 128)
     # 0.73 of their time; with a CTA of 512 threads for every 1024 nodes 1.07
     assert t["1"] <= 0.9 * t["0"]
+
+
+def test_a_tall_narrow_grid_takes_no_longer_than_a_wide_flat_one():
+    # 0.8 of its time; with whole columns only 2.2 times
+    assert _best_ms(32, 16384) <= 1.3 * _best_ms(16384, 32)
