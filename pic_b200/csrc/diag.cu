@@ -237,11 +237,17 @@ __device__ __forceinline__ int x_bin(double X, int nbins) {
 // so a run stays within one x column, or two neighbours where a column's edge
 // (one Debye length, about one cell) crosses the cells, for a long time: the
 // lanes sum those two columns (base, base + 1) in registers and the warp adds
-// them to the CTA's shared sums only when a batch has left them.  Lanes
-// outside the two (unsorted particles) add their own.  HBM-bound in aim (36 B
-// a particle FP64); 104 -> 53 us (pass 1) and 112 -> 63 us (pass 2) for 5.7M
-// particles against shuffled warp sums of every 32 particles.
+// them to the CTA's shared sums only when a batch has left them.  HBM-bound in
+// aim (36 B a particle FP64).  Both passes of a call, 5.2 to 5.7M FP64
+// particles (us: warp sums of every 32 particles; two columns that moved at
+// every lane outside, which added its own; now):
+//   sorted, cells of half a column, 500 columns           262   185   184
+//   ten steps after the sort                              553   568   247
+//   random order, 500 columns / 64 columns            258/713 327/838 237/505
+//   sorted, cells of 1.9 columns, 500 / 8 columns     524/280 480/388 241/214
+// (the last: colliding adds, in the few warps that have them as long as all)
 constexpr int kMomBatch = 2;  // particles a lane has in flight
+constexpr int kMomShare = 4;  // lanes outside in one column whose values the warp sums
 
 template <bool kSecond, bool F32>
 __global__ void __launch_bounds__(256, 4) k_vmoments(MomK k) {
@@ -319,11 +325,7 @@ __global__ void __launch_bounds__(256, 4) k_vmoments(MomK k) {
       // the two columns move on to the lowest of the batch where the new two
       // hold every live lane, or most of them with most of them gone from the
       // old: a run of sorted particles that crosses into its next column.
-      // Particles in no order have no such pair.  Both passes of 5.2M
-      // particles, 500 columns, against warp sums of every 32 particles and
-      // against moving at every lane that left: sorted 262, 185 -> 184 us; ten
-      // steps after the sort 553, 568 -> 373; random order 258, 327 -> 232 (with
-      // 64 columns, where the shared adds of one column collide: 713, 838 -> 751)
+      // Particles in no order have no such pair.
       const unsigned left = __ballot_sync(full, b[u] >= 0 && b[u] != base && b[u] != base + 1);
       if (left) {
         const int live = __popc(__ballot_sync(full, b[u] >= 0));
@@ -346,12 +348,39 @@ __global__ void __launch_bounds__(256, 4) k_vmoments(MomK k) {
       }
       c0 += in0 ? 1u : 0u;
       c1 += in1 ? 1u : 0u;
-      if (b[u] >= 0 && !in0 && !in1) {
+      // the lanes outside: columns that several of them share (cells wider than
+      // a column or two) as one sum of the warp, the others on their own
+      unsigned out = __ballot_sync(full, b[u] >= 0 && !in0 && !in1);
+      if (out) {
+        const bool mine = out >> lane & 1;
+        double t[3];
+#pragma unroll
         for (int c = 0; c < 3; ++c) {
-          const double d = kSecond ? v[u][c] - dr[c * k.nbins + b[u]] : 0.0;
-          atomicAdd(&acc[c * k.nbins + b[u]], kSecond ? d * d : v[u][c]);
+          const double d = kSecond && mine ? v[u][c] - dr[c * k.nbins + b[u]] : 0.0;
+          t[c] = kSecond ? d * d : v[u][c];
         }
-        if (!kSecond) atomicAdd(&cnt[b[u]], 1u);
+        while (out) {
+          const int first = __ffs(out) - 1, col = __shfl_sync(full, b[u], first);
+          const unsigned share = __ballot_sync(full, b[u] == col);
+          if (__popc(share) < kMomShare) break;
+          double a[3];
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            a[c] = share >> lane & 1 ? t[c] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) a[c] += __shfl_xor_sync(full, a[c], o);
+          }
+          if (lane == first) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) atomicAdd(&acc[c * k.nbins + col], a[c]);
+            if (!kSecond) atomicAdd(&cnt[col], (unsigned)__popc(share));
+          }
+          out &= ~share;
+        }
+        if (out >> lane & 1) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) atomicAdd(&acc[c * k.nbins + b[u]], t[c]);
+          if (!kSecond) atomicAdd(&cnt[b[u]], 1u);
+        }
       }
     }
   }
