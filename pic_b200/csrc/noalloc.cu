@@ -77,33 +77,41 @@ __device__ __forceinline__ void na_add(unsigned long long *acc, int n1, int nny,
 // needs are products (div_dev.h, the same bits as the divisions).
 // A call with those particles: 158 -> 38 us.
 constexpr int kNaRun = 4;
+// One particle a thread while a wave of them holds all: the latency of one counts
+// (30,001 on 257 x 200 nodes: four each 22.6 us a call, one 20.3, sorted ones too);
+// and while there are less than two particles a node, so hardly a run (600,000
+// on 700 x 700: 32.6, one each 30.6).
+constexpr int64_t kNaFew = 148 * 2048;
 
+template <int RUN>
 __global__ void __launch_bounds__(256) k_na_deposit(int nnx, int nny, double xmin, double ymin, double hx, double hy,
                                                     int64_t n, const double *__restrict__ x,
                                                     const double *__restrict__ y, const int32_t *__restrict__ loc,
                                                     int vec, unsigned long long *acc) {
-  const int64_t p0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kNaRun;
+  const int64_t p0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * RUN;
   const int nex = nnx - 1, ney = nny - 1, lane = threadIdx.x & 31;
-  const double rhx = pic::recip_const(hx), rhy = pic::recip_const(hy);
-  double px[kNaRun], py[kNaRun];
-  int lc[kNaRun];
-  if (vec && p0 + kNaRun <= n) {  // 16-byte aligned arrays
+  const double rhx = RUN > 1 ? pic::recip_const(hx) : 0.0, rhy = RUN > 1 ? pic::recip_const(hy) : 0.0;
+  double px[RUN], py[RUN];
+  int lc[RUN];
+  if (RUN > 1 && vec && p0 + RUN <= n) {  // 16-byte aligned arrays
+    if constexpr (RUN > 1) {
 #pragma unroll
-    for (int k = 0; k < kNaRun; k += 2) {
-      const double2 a = *reinterpret_cast<const double2 *>(x + p0 + k), b = *reinterpret_cast<const double2 *>(y + p0 + k);
-      px[k] = a.x;
-      px[k + 1] = a.y;
-      py[k] = b.x;
-      py[k + 1] = b.y;
+      for (int k = 0; k < RUN; k += 2) {
+        const double2 a = *reinterpret_cast<const double2 *>(x + p0 + k), b = *reinterpret_cast<const double2 *>(y + p0 + k);
+        px[k] = a.x;
+        px[k + 1] = a.y;
+        py[k] = b.x;
+        py[k + 1] = b.y;
+      }
+      const int4 l = loc ? *reinterpret_cast<const int4 *>(loc + p0) : make_int4(0, 0, 0, 0);
+      lc[0] = l.x;
+      lc[1] = l.y;
+      lc[2] = l.z;
+      lc[3] = l.w;
     }
-    const int4 l = loc ? *reinterpret_cast<const int4 *>(loc + p0) : make_int4(0, 0, 0, 0);
-    lc[0] = l.x;
-    lc[1] = l.y;
-    lc[2] = l.z;
-    lc[3] = l.w;
   } else {
 #pragma unroll
-    for (int k = 0; k < kNaRun; ++k) {
+    for (int k = 0; k < RUN; ++k) {
       const bool in = p0 + k < n;
       px[k] = in ? x[p0 + k] : 0.0;
       py[k] = in ? y[p0 + k] : 0.0;
@@ -113,10 +121,14 @@ __global__ void __launch_bounds__(256) k_na_deposit(int nnx, int nny, double xmi
   int key = -1;  // the run's first node
   long long q[4] = {0, 0, 0, 0};
 #pragma unroll
-  for (int k = 0; k < kNaRun; ++k) {
+  for (int k = 0; k < RUN; ++k) {
     if (lc[k] < 0) continue;  // absorbed slot
-    bool exact = true;
-    double rxp = pic::div_const(px[k] - xmin, hx, rhx, exact), ryp = pic::div_const(py[k] - ymin, hy, rhy, exact);
+    bool exact = RUN > 1;  // one particle a thread: the divisions are the shorter chain
+    double rxp = 0.0, ryp = 0.0;
+    if (RUN > 1) {
+      rxp = pic::div_const(px[k] - xmin, hx, rhx, exact);
+      ryp = pic::div_const(py[k] - ymin, hy, rhy, exact);
+    }
     if (!exact) {
       rxp = (px[k] - xmin) / hx;
       ryp = (py[k] - ymin) / hy;
@@ -128,9 +140,12 @@ __global__ void __launch_bounds__(256) k_na_deposit(int nnx, int nny, double xmi
     const int ie = i - 1, je = j - 1;
     const double x1 = xmin + hx * ie, x2 = xmin + hx * (ie + 1);
     const double y1 = ymin + hy * je, y2 = ymin + hy * (je + 1);
-    exact = true;
-    double dx = pic::div_const(px[k] - x1, x2 - x1, pic::recip_near(x2 - x1, rhx), exact);
-    double dy = pic::div_const(py[k] - y1, y2 - y1, pic::recip_near(y2 - y1, rhy), exact);
+    exact = RUN > 1;
+    double dx = 0.0, dy = 0.0;
+    if (RUN > 1) {
+      dx = pic::div_const(px[k] - x1, x2 - x1, pic::recip_near(x2 - x1, rhx), exact);
+      dy = pic::div_const(py[k] - y1, y2 - y1, pic::recip_near(y2 - y1, rhy), exact);
+    }
     if (!exact || fabs((x2 - x1) - hx) > 1e-9 * hx || fabs((y2 - y1) - hy) > 1e-9 * hy) {
       dx = (px[k] - x1) / (x2 - x1);
       dy = (py[k] - y1) / (y2 - y1);
@@ -217,10 +232,11 @@ extern "C" int pic_deposit_noalloc(int32_t nnx, int32_t nny, double xmin, double
   cudaStream_t st = (cudaStream_t)stream;
   const double hx = (xmax - xmin) / (nnx - 1), hy = (ymax - ymin) / (nny - 1);
   k_na_clear<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, nn);
-  if (n > 0)
-    k_na_deposit<<<(unsigned)((n + 256 * kNaRun - 1) / (256 * kNaRun)), 256, 0, st>>>(
-        nnx, nny, xmin, ymin, hx, hy, n, x, y, loc,
-        (((uintptr_t)x | (uintptr_t)y | (uintptr_t)loc) & 15) == 0, acc);
+  if (n > 0) {
+    const int run = n <= kNaFew || n < 2 * nn ? 1 : kNaRun;
+    (run == 1 ? k_na_deposit<1> : k_na_deposit<kNaRun>)<<<(unsigned)((n + 256 * run - 1) / (256 * run)), 256, 0, st>>>(
+        nnx, nny, xmin, ymin, hx, hy, n, x, y, loc, (((uintptr_t)x | (uintptr_t)y | (uintptr_t)loc) & 15) == 0, acc);
+  }
   k_na_normalize<<<(unsigned)((nn + 255) / 256), 256, 0, st>>>(acc, cell_volume, weight_charge, L_ref, n_ref,
                                                                 rho_out, nn);
   e = cudaGetLastError();
