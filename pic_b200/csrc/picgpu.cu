@@ -1493,11 +1493,12 @@ __device__ __forceinline__ double row_apply(const PcgK &k, int64_t n, F v) {
       for (int c = 0; c < 3; ++c) acc = fma(c_stencil[kind][3 * a + c], v(base + (int64_t)a * k.nny + c), acc);
   } else if (EX == 1 || (EX == 2 && k.st_tab)) {
     const bool edge = n < k.nny + 1 || n >= k.nn - k.nny - 1;
+    const double *tab = k.st_tab + kind * k.st_rs;
     double val[9], xv[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) val[q] = k.st_tab[q * k.st_cs + kind * k.st_rs];
-#pragma unroll
     for (int q = 0; q < 9; ++q) xv[q] = v(stencil_node(k, n, edge, q));
+#pragma unroll
+    for (int q = 0; q < 9; ++q) val[q] = tab[q * k.st_cs];
 #pragma unroll
     for (int q = 0; q < 9; ++q) acc = fma(val[q], xv[q], acc);
   } else {
@@ -1789,6 +1790,7 @@ __device__ __forceinline__ void final_sum_wide(const double *part, int nb, doubl
   __syncthreads();
 }
 
+template <int EX>  // explicit rows as lists (0) or stencils (1): with both, registers spilled (2 to 3% of an iteration)
 __global__ void __launch_bounds__(kWide, 1) k_pcg_persist(PcgP P) {
   const PcgK &k = P.k;
   PcgState *S = k.st;
@@ -1815,7 +1817,7 @@ __global__ void __launch_bounds__(kWide, 1) k_pcg_persist(PcgP P) {
       double pv = 0.0, qv = 0.0;
       if (threadIdx.x < nvalid) {
         pv = pn(n);
-        qv = row_apply(k, n, pn);
+        qv = row_apply<EX>(k, n, pn);
         pnew[n] = pv;
         k.q[n] = qv;
       }
@@ -3937,6 +3939,11 @@ static int run_rhs() {
   return PIC_OK;
 }
 
+// the persistent PCG for this context's explicit rows
+static const void *pcg_fn() {
+  return g.ex_stencil ? (const void *)k_pcg_persist<1> : (const void *)k_pcg_persist<0>;
+}
+
 // The on-chip PCG built for the chunks a CTA owns at most: a group of 256
 // threads a chunk while four groups do, then two chunks a group.
 struct SmemPcg {
@@ -4011,7 +4018,7 @@ static int run_pcg(pic_solve_stats *stats) {
       PIC_CUDA(cudaLaunchCooperativeKernel(v.fn, dim3(g.smem_grid), dim3(v.threads), args, g.smem_bytes, g.st));
     } else {
       void *args[] = {&P};
-      PIC_CUDA(cudaLaunchCooperativeKernel((const void *)k_pcg_persist, dim3(g.coop_grid), dim3(kWide),
+      PIC_CUDA(cudaLaunchCooperativeKernel(pcg_fn(), dim3(g.coop_grid), dim3(kWide),
                                            args, 0, g.st));
     }
     PIC_LAUNCHED();
@@ -5330,7 +5337,7 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     PIC_CUDA(cudaGetDevice(&dev));
     PIC_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     PIC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_persist, kWide, 0));
+    PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pcg_fn(), kWide, 0));
     const char *env = getenv("PIC_PCG_PERSISTENT");
     bool want = !(env && env[0] == '0');
     g.coop_grid = (want && coop && per_sm > 0) ? std::min(g.red_blocks, per_sm * nsm) : 0;
