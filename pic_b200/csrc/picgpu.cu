@@ -5385,7 +5385,16 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
     PIC_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     const int cpc = (g.red_blocks + nsm - 1) / nsm;
     const SmemPcg v = smem_pcg(cpc);
-    if (want_smem && coop && g.ex_local && cpc <= 2 * kPcgMaxGroups && v.bytes + 4096 <= (size_t)max_smem) {
+    // Every CTA polls a column and a half of neighbours' values on each side an
+    // iteration: few rounds where a thread has few of them, more than the chunked
+    // kernel's two grid barriers where the columns are long for the CTA (us an
+    // iteration, chunked -> on-chip: 1 chunk a CTA, 20 x 2500 nodes 10.9 -> 10.1,
+    // 20 x 3000 11.4 -> 11.6, 20 x 6000 11.0 -> 19.0; 2 chunks, 60 x 4500 14.4 ->
+    // 12.5, 30 x 5000 11.8 -> 14.1; 3 and 4, 60 x 5000 16.0 -> 15.6, 60 x 6000 17.2 -> 17.6)
+    const int halo = 2 * (m.nny + 1) / v.threads;  // of a thread
+    const bool short_strips = halo < (cpc <= 1 ? 20 : cpc <= 2 ? 18 : 11);
+    if (want_smem && coop && g.ex_local && short_strips && cpc <= 2 * kPcgMaxGroups &&
+        v.bytes + 4096 <= (size_t)max_smem) {
       PIC_CUDA(cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.bytes));
       int per_sm2 = 0;
       PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm2, v.fn, v.threads, v.bytes));

@@ -49,3 +49,22 @@ def test_persistent_matches_two_kernels(name, ncx, ncy, swap, monkeypatch):
     b = _solve(monkeypatch, name, ncx, ncy, {"PIC_PCG_PERSISTENT": "0"}, swap)
     assert a[:2] == b[:2] and a[1] == 0 and a[0] > 3
     assert np.array_equal(a[3], b[3])
+
+
+# columns at the length where each number of chunks a CTA hands over to the
+# chunked kernel (2 (nny + 1) halo values for 256, 512 and 1024 threads)
+@pytest.mark.parametrize("ncx,ncy", [(12, 2557), (12, 2558), (40, 4605), (40, 4606), (70, 5629), (70, 5630)])
+def test_long_columns_match_the_chunked_kernel(ncx, ncy, monkeypatch):
+    a = _solve(monkeypatch, "tiny", ncx, ncy, {})
+    b = _solve(monkeypatch, "tiny", ncx, ncy, {"PIC_PCG_SMEM": "0"})
+    assert a[:2] == b[:2] and a[1] == 0 and a[0] > 3
+    assert np.array_equal(a[3], b[3])
+
+
+def test_long_columns_take_no_longer_than_in_the_chunked_kernel(monkeypatch):
+    t = {}
+    for mode in ("default", "0"):
+        env = {} if mode == "default" else {"PIC_PCG_SMEM": "0"}
+        t[mode] = min(_solve(monkeypatch, "tiny", 20, 6000, env)[2] for _ in range(4))
+    # on chip 1.7 times
+    assert t["default"] <= 1.25 * t["0"]
