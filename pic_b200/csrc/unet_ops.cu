@@ -809,8 +809,12 @@ int unet_wgrad(int32_t n, int32_t h, int32_t w, int32_t c, int32_t k, const void
   if (n < 1 || h < 1 || w < 1 || c < 1 || k < 1) return UNET_ERR_SHAPE;
   const int64_t np = (int64_t)n * h * w;
   // the tensor-core form wants 16-byte channel groups (and indexes tiles in
-  // 32 bits); other shapes and alignments take the CUDA cores
-  if (c % 8 == 0 && k % 8 == 0 && (((uintptr_t)x | (uintptr_t)dy) & 15) == 0 && np < ((int64_t)1 << 31)) {
+  // 32 bits); other shapes and alignments take the CUDA cores, and so do images
+  // that leave nearly all of a tile empty, one pixel wide or of two in all
+  // (100,000 pixels of 32 -> 32 channels, CUDA cores and tensor cores, us: 1x1
+  // 273, 671; 2x1 282, 411; 1x2 284, 339; 6x1 282, 385; 16x1 280, 292)
+  if (c % 8 == 0 && k % 8 == 0 && (((uintptr_t)x | (uintptr_t)dy) & 15) == 0 && np < ((int64_t)1 << 31) && w > 1 &&
+      (int64_t)h * w > 2) {
     if (k > 32) return run_wgrad_mma<4>(n, h, w, c, k, (const bf16 *)x, (const bf16 *)dy, dw, (cudaStream_t)stream);
     return run_wgrad_mma<2>(n, h, w, c, k, (const bf16 *)x, (const bf16 *)dy, dw, (cudaStream_t)stream);
   }
