@@ -424,12 +424,13 @@ PartK part_k(const Species &s) {
 // CTAs of one wave (all resident at once), fewer for few particles
 template <class K>
 int grid_for(K kernel, size_t smem, int64_t n, unsigned *grid) {
-  int dev = 0, nsm = 0, per_sm = 0;
+  int dev = 0, nsm = 0, per_sm = 1;
   PIC_CUDA(cudaGetDevice(&dev));
   PIC_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   PIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem));
-  *grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(blocks_for(n, 256), (int64_t)nsm * std::max(per_sm, 1)));
+  const int64_t all = blocks_for(n, 256);
+  if (all > nsm) PIC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem));
+  *grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(all, (int64_t)nsm * std::max(per_sm, 1)));
   return PIC_OK;
 }
 
