@@ -5055,19 +5055,6 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
       const int64_t c = d - (int64_t)a * nny;
       return c < -1 || c > 1 || (c < 0 && j == 0) || (c > 0 && j == nny - 1) ? -1 : 3 * (a + 1) + (int)c + 1;
     };
-    for (int i = 0; i < m.nnx && as_stencil; ++i)
-      for (int j = 0; j < nny && as_stencil; ++j) {
-        const int64_t n = (int64_t)i * nny + j;
-        const int u = mesh->node_type[n];
-        if (u <= 0) continue;
-        int last = -1;
-        for (int64_t q = mesh->a_srow[u - 1] - 1; q < mesh->a_srow[u] - 1; ++q) {
-          const int at = position(u2n[mesh->a_jcol[q] - 1] - n, j);
-          as_stencil = as_stencil && at > last;
-          last = at;
-        }
-      }
-    g.ex_stencil = as_stencil;
     std::vector<std::array<double, 9>> st_rows;
     std::unordered_map<std::string, int32_t> st_index;
     std::vector<int32_t> kind(nn, -1), ex_cnt, ex_col;
@@ -5104,7 +5091,20 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
         if (as_stencil) {
           std::array<double, 9> S;
           S.fill(0.0);
-          for (auto &pr : ent) S[position(pr.first - n, j)] = pr.second;
+          int last = -1;
+          for (auto &pr : ent) {
+            const int at = position(pr.first - n, j);
+            as_stencil = as_stencil && at > last;
+            if (at >= 0) S[at] = pr.second;
+            last = at;
+          }
+          if (!as_stencil) {  // from the start again, as lists
+            st_rows.clear();
+            st_index.clear();
+            std::fill(kind.begin(), kind.end(), -1);
+            n = -1;
+            continue;
+          }
           // the previous column's row at this radius, mostly, on r-z meshes
           const int32_t before = i > 0 ? kind[n - nny] - g.n_mat : -1;
           if (before >= 0 && std::memcmp(st_rows[before].data(), S.data(), sizeof S) == 0) {
@@ -5126,6 +5126,7 @@ int pic_init(const pic_mesh_desc *mesh, const pic_params *params) {
         }
       }
     }
+    g.ex_stencil = as_stencil;
     PIC_CUDA(cudaMemcpyToSymbol(c_stencil, g.h_stencil, sizeof g.h_stencil));
     {
       float st32[16][9];
