@@ -135,7 +135,7 @@ struct Ctx {
   bool ex_stencil = true;
   int2 *d_fcg_rows = nullptr;      // per CTA of the persistent FCG: kinds of its explicit rows
   size_t fcg_tab_bytes = 0;        // shared memory they take
-  float *d_fcg32 = nullptr;        // mixed-precision FCG: 11 FP32 vectors, allocated on first use
+  float *d_fcg32 = nullptr;        // mixed-precision FCG: nine FP32 vectors, allocated on first use
   int fcg_inner32 = 0;             // mixed precision: FP32 inner FCG in FP64 refinement (pic_set_fcg_inner)
   int n_mat = 0;
   double h_stencil[16][9];

@@ -2731,7 +2731,7 @@ struct FcgP {
   // zF shares t's buffer (t is dead once it is restricted) and Q is one
   // buffer (its old values are read by their own node only when it is
   // rewritten): the vectors of a 1024^2 solve then stay in L2
-  V *zA, *t, *zF, *P0, *P1, *Q0, *Q1;
+  V *zA, *t, *zF, *P0, *P1, *Q;
   double *part;                  // [4][grid] partials: F p.q, F p.r, A r.r, E zF.Q
   const __half *ainv;            // coarse inverse / ainv_scale, rows padded to ainv_ld (a multiple of 8)
   double ainv_scale;
@@ -3090,14 +3090,14 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
   }
   for (;;) {
     // the previous direction (written last iteration), the new one
-    const V *Pl = parity ? F.P0 : F.P1, *Ql = parity ? F.Q0 : F.Q1;
-    V *Pn = parity ? F.P1 : F.P0, *Qn = parity ? F.Q1 : F.Q0;
+    const V *Pl = parity ? F.P0 : F.P1;
+    V *Pn = parity ? F.P1 : F.P0, *Q = F.Q;
     // (A) update with the previous direction, then pre-smoothing
     {
-      const V *r = rc_, *Qp = Ql;
+      const V *r = rc_;
       const V a = (V)alpha;
       const bool upd = have_old;
-      auto rnew = [&](int64_t m) { return upd ? vfma(-a, Qp[m], r[m]) : r[m]; };
+      auto rnew = [&](int64_t m) { return upd ? vfma(-a, Q[m], r[m]) : r[m]; };
       double acc_rr = 0.0;
       auto node_a = [&](int64_t n) {
         const V rv = rnew(n);
@@ -3120,7 +3120,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
         struct Pre { V x, p; int kind; };
         march<V>(
             F.nnx, k.nny, own,
-            [&](unsigned m, int, int) { return Raw{at(r, m), upd ? at(Qp, m) : (V)0, at(F.dinv, m)}; },
+            [&](unsigned m, int, int) { return Raw{at(r, m), upd ? at(Q, m) : (V)0, at(F.dinv, m)}; },
             [&](const Raw &v) { return (om * (upd ? vfma(-a, v.q, v.r) : v.r)) * v.d; },
             [&](unsigned n) { return Pre{upd ? at(F.x, n) : (V)0, upd ? at(Pl, n) : (V)0, at(k.row_kind, n)}; },
             [&](unsigned n, const V(&w)[3][3], const Raw &v, const Pre &p) {
@@ -3255,7 +3255,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
         }
       if (!(ok = barrier())) break;
     }
-    // (E) post-smoothing of zA + P e_1 and zF.Q_old (Q_old is this iteration's Ql)
+    // (E) post-smoothing of zA + P e_1 and zF.Q_old (Q_old is this iteration's Q)
     {
       double acc_zq = 0.0;
       auto put_e = [&](unsigned n, V zf, V q) {
@@ -3275,7 +3275,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
         auto eval = [&](const Raw &v) { return v.kind < 0 ? (V)0 : mgrid ? (V)((double)v.z + v.pe) : v.z; };
         march<V>(
             F.nnx, k.nny, own, load, eval,
-            [&](unsigned n) { return Pre{at(F.dinv, n), at(r, n), have_old ? at(Ql, n) : (V)0}; },
+            [&](unsigned n) { return Pre{at(F.dinv, n), at(r, n), have_old ? at(Q, n) : (V)0}; },
             [&](unsigned n, const V(&w)[3][3], const Raw &v, const Pre &p) {
               put_e(n, v.kind < 0 ? (V)0 : vfma(om * p.d, p.r - stencil9<V>(k, tab, v.kind, w), w[1][1]), p.q);
             },
@@ -3285,7 +3285,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
                 auto za = [&](int64_t m) { return eval(load((unsigned)m, (int)m / k.nny, (int)m % k.nny)); };
                 zf = vfma(om * F.dinv[n], r[n] - row_apply_v<V, EX>(k, n, za), za(n));
               }
-              put_e((unsigned)n, zf, have_old ? Ql[n] : (V)0);
+              put_e((unsigned)n, zf, have_old ? Q[n] : (V)0);
             });
       } else {
         for (int64_t n = n0 + threadIdx.x; n < n1; n += kFcgT) {
@@ -3294,7 +3294,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
             auto za = [&](int64_t m) { return F.zA[m]; };
             zf = vfma(om * F.dinv[n], r[n] - row_apply_v<V, EX>(k, n, za), za(n));
           }
-          put_e((unsigned)n, zf, have_old ? Ql[n] : (V)0);
+          put_e((unsigned)n, zf, have_old ? Q[n] : (V)0);
         }
       }
       double v[1] = {acc_zq}, o[1];
@@ -3318,7 +3318,7 @@ __global__ void __launch_bounds__(kFcgT, 1) k_fcg_persist(FcgP<V> F) {
       double acc[2] = {0.0, 0.0};
       auto put_f = [&](unsigned n, V pv, V qv, V rv) {
         at(Pn, n) = pv;
-        at(Qn, n) = qv;
+        at(Q, n) = qv;
         acc[0] = fma((double)pv, (double)qv, acc[0]);
         acc[1] = fma((double)pv, (double)rv, acc[1]);
       };
@@ -4260,8 +4260,7 @@ static int run_fcg_persist64(pic_solve_stats *stats, int *fcg_iters, int *rc_out
   F.zF = g.d_pc_t;
   F.P0 = g.d_fcg_P;
   F.P1 = g.d_fcg_P + nn;
-  F.Q0 = g.d_fcg_Q;
-  F.Q1 = g.d_fcg_Q;
+  F.Q = g.d_fcg_Q;
   const void *fn = fcg_fn<double>();
   const size_t smem = (size_t)g.pc_ainv_ld * sizeof(double) + g.fcg_tab_bytes;  // coarse_gemv's staging, explicit rows
   F.tab_rows = g.d_fcg_rows;
@@ -4419,8 +4418,8 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
       // Mixed precision: FP32 inner FCG solves of A e = r inside FP64 iterative
       // refinement (x += e, r = b - A x in FP64, tested against the tolerance).
       if (!g.d_fcg32) {
-        if ((rc = dalloc(&g.d_fcg32, 11 * (size_t)nn))) { *rc_out = rc; return 1; }
-        k_f64_to_f32<<<nb, 256, 0, g.st>>>(g.d_pc_dinv, g.d_fcg32 + 10 * (size_t)nn, nn);
+        if ((rc = dalloc(&g.d_fcg32, 9 * (size_t)nn))) { *rc_out = rc; return 1; }
+        k_f64_to_f32<<<nb, 256, 0, g.st>>>(g.d_pc_dinv, g.d_fcg32 + 8 * (size_t)nn, nn);
         PIC_LAUNCHED();
       }
       float *v32 = g.d_fcg32;
@@ -4432,11 +4431,10 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
       F.zA = v32 + 3 * nn;
       F.t = v32 + 4 * nn;
       F.zF = v32 + 4 * nn;
-      F.P0 = v32 + 6 * nn;
-      F.P1 = v32 + 7 * nn;
-      F.Q0 = v32 + 8 * nn;
-      F.Q1 = v32 + 8 * nn;
-      F.dinv = v32 + 10 * nn;
+      F.P0 = v32 + 5 * nn;
+      F.P1 = v32 + 6 * nn;
+      F.Q = v32 + 7 * nn;
+      F.dinv = v32 + 8 * nn;
       int outer = 0, total = 0;
       for (;;) {
         if (hs.rr / hs.rhs <= hs.tol2) {
@@ -4494,8 +4492,7 @@ static int run_fcg(pic_solve_stats *stats, int *fcg_iters, int *rc_out) {
     F.zF = g.d_pc_t;
     F.P0 = g.d_fcg_P;
     F.P1 = g.d_fcg_P + nn;
-    F.Q0 = g.d_fcg_Q;
-    F.Q1 = g.d_fcg_Q;
+    F.Q = g.d_fcg_Q;
     for (;;) {
       if ((rc = launch(F, fcg_fn<double>()))) { *rc_out = rc; return 1; }
       PIC_CUDA(cudaMemcpyAsync(&hs, g.d_fcg, sizeof hs, cudaMemcpyDeviceToHost, g.st));
