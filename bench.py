@@ -61,8 +61,8 @@ MIXED_PUSH_BYTES_RZ = 48
 # the 1024^2 eight-ellipse deck at 8 particles per cell (FP64 k_push_bulk,
 # mixed k_push_mixed_bulk) and the 2048x1024 r-z deck at 8 (mixed r-z);
 # "_sel": the push also builds the MCC selection (reads the ids)
-NCU_PUSH_TRAFFIC = {"fp64": 68.0, "mixed": 38.0, "mixed_rz": 51.4,
-                    "fp64_sel": 72.2, "mixed_sel": 42.4, "mixed_rz_sel": 55.5}
+NCU_PUSH_TRAFFIC = {"fp64": 68.0, "mixed": 38.1, "mixed_rz": 51.6,
+                    "fp64_sel": 72.2, "mixed_sel": 43.1, "mixed_rz_sel": 57.2}
 
 
 def _dist():

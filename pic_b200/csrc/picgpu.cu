@@ -1026,8 +1026,6 @@ __global__ void __launch_bounds__(256, 4) k_push_tiled(MeshK m, FieldK f, PushK 
   cp_async_wait<0>();
 }
 
-// FP64 absolute particles (staging set) -> FP32 offsets inside the located
-// element and FP32 velocities (live set).  Slots with loc < 0 are copied as 0.
 // FP64 push with bulk-copied tiles: one thread issues five 1-D
 // cp.async.bulk copies per 256-particle tile (x, y, vx, vy: 2 KB each; the
 // elements: 1 KB), which complete on the stage's mbarrier; the other threads
@@ -1146,10 +1144,13 @@ __global__ void __launch_bounds__(256, MINB) k_push_bulk(MeshK m, FieldK f, Push
 }
 
 // The mixed-precision push with bulk-copied tiles (elements and FP32
-// offsets and velocities: five 1 KB copies a tile), as k_push_bulk, but both
-// particles of a pair in flight at once: 64 registers, 8 CTAs of 128 threads
-// (one after the other at 48 registers and 10 CTAs: spills).  Against one a
-// thread: 0.310 -> 0.299 ms for 14.3M particles, r-z 1.89 -> 1.70 ms for 66.8M.
+// offsets and velocities: five 1 KB copies a tile), as k_push_bulk, but a
+// thread takes two consecutive particles, both in flight at once and pushed in
+// place in the tile, and hands them to one pair_deposit, whose segmented warp
+// sums were the largest part of the instructions that bound it: 64 registers,
+// 8 CTAs of 128 threads (one particle after the other at 48 registers and 10
+// CTAs: spills).  Against one a thread: 0.319 -> 0.305 ms for 14.5M particles,
+// r-z 1.89 -> 1.69 ms for 66.9M.
 __device__ __forceinline__ void push_tile_bulk(PushTile *T, uint64_t *b, const SpK &s, int64_t base) {
   mbar_expect_tx(b, (unsigned)sizeof(PushTile));
   bulk_g2s(T->loc, s.loc + base, 4 * kPushTile, b);
@@ -1264,6 +1265,8 @@ __global__ void __launch_bounds__(kPairThreads, MINB) k_push_mixed_bulk(MeshK m,
   push_select_flush(s, sel_buf);
 }
 
+// FP64 absolute particles (staging set) -> FP32 offsets inside the located
+// element and FP32 velocities (live set).  Slots with loc < 0 are copied as 0.
 __global__ void k_to_mixed(MeshK m, const double *__restrict__ x, const double *__restrict__ y,
                            const double *__restrict__ vx, const double *__restrict__ vy,
                            const double *__restrict__ vz, const int32_t *__restrict__ loc, float *__restrict__ ox,
@@ -4027,7 +4030,7 @@ static int run_pcg(pic_solve_stats *stats) {
     if (g.smem_grid > 0) g.pcg_tag += (unsigned)hs.iter + 2;  // every tag this solve can have published
     if (hs.ierr == 4) {
       if (int rc_ = pcg_slots_clear()) return rc_;
-      set_error("pic_ife_solve: PCG grid barrier timed out");
+      set_error("pic_ife_solve: PCG wait for another CTA timed out");
       return PIC_ERR_CUDA;
     }
   }
